@@ -85,8 +85,20 @@ StepArgs make_args(tslb_ctx* c, const void* in, void* out) {
     StepArgs a;
     std::memset(&a, 0, sizeof(a));
     a.nx = c->nx; a.ny = c->ny; a.nz = c->nz; a.N = c->N;
+    a.plane = (unsigned)c->nx * (unsigned)c->ny;
     a.in = in; a.out = out; a.nrm = c->nrm;
+    for (int f = 0; f < NF; ++f) {
+        a.fi[f] = static_cast<const char*>(in) + (size_t)f * c->N * c->esize;
+        a.fo[f] = static_cast<char*>(out) + (size_t)f * c->N * c->esize;
+    }
     a.zchunk = c->zchunk;
+    a.warps = c->warps;
+    a.grid = c->grid;
+    a.th = c->th;
+    a.xwrap = c->p.bc[0] == TSLB_BC_PERIODIC && c->nx <= 32;
+    a.phi_mirror = c->p.wall_phi_mode != 0;
+    for (int f = 0; f < 6; ++f)
+        if (c->p.bc[f] == TSLB_BC_INLET) a.phi_mirror = 0;
     a.zt0 = c->zt0;
     a.zt1 = c->zt1 > 0 ? c->zt1 : c->nz;
     a.zoff = c->z_begin - c->zt0;
@@ -597,38 +609,54 @@ int ensure_normals(tslb_ctx* c) {
     return TSLB_OK;
 }
 
-// tile columns of the step grid
-long long step_tiles(int nx, int ny) { return (long long)((nx + TX - 1) / TX) * ((ny + TY - 1) / TY); }
-constexpr int kStepBlocksPerSM = 2;   // resident step blocks per SM (registers and shared memory)
+// How the step kernel cuts a lattice: warps of a block, target rows of a tile,
+// target planes of a block (0: `grid` blocks share the tiles' planes equally).
+struct StepPlan { int warps, th, zchunk, grid; };
+constexpr int kEnsBlocksPerSM = BIGW / SMALLW;   // ensemble blocks (SMALLW warps) resident on an SM
 
-// Target planes per block.  Each chunk also reads the source planes just
-// outside it, so long chunks repeat less work; the chunks per tile column
-// are the fewest whose blocks fill the resident slots (bps blocks per SM) in
-// whole waves to at least 90%, with chunks of at least 8 planes.
-int choose_zchunk(long long tiles, int nz, int sms, int bps, int mode) {
-    const long long slots = (long long)bps * sms;
-    const int max_chunks = std::max(1, nz / 8);
-    int best = 1;
-    double best_fill = -1.0;
-    for (int nc = 1; nc <= max_chunks; ++nc) {
-        const int zc = (nz + nc - 1) / nc;
-        const long long blocks = tiles * ((nz + zc - 1) / zc);
-        const long long waves = (blocks + slots - 1) / slots;
-        const double fill = (double)blocks / (double)(waves * slots);
-        if (fill > best_fill + 1e-9) {
-            best_fill = fill;
-            best = nc;
+int even_rows(int ny, int most) {   // tiles of equal height, at most `most` rows
+    const int tiles = (ny + most - 1) / most;
+    return (ny + tiles - 1) / tiles;
+}
+
+// The plan with the least estimated time, in microseconds on a B200.  A block
+// takes `plane` per source plane and about `extra` planes' time outside its
+// target planes (two more source planes, its start); blocks run in waves.
+// Measured on the 384 x 192 x 128 colour channel: 16-warp blocks in 32 / 16 / 8
+// plane chunks 0.350 / 0.379 / 0.442 ms, which is 2.0 us a plane and 3 planes
+// extra; two 8-warp blocks on an SM 1.72 us a plane, of fewer rows (6 of 8 are
+// targets, against 14 of 16).  Equal shares have no last wave, but their blocks
+// are at different planes and share less of what they read: 8% slower a plane
+// (0.373 ms on the channel, where chunks fill 4.92 waves; 52 against 58 us on a
+// 173 x 59 x 91 Couette cell).  The phase field takes chunks only, and short
+// ones: planes with interface nodes are about three times slower, so the last
+// blocks to finish are those across a droplet, by their length (96^3 with one
+// droplet: 130 us in 24-plane chunks).
+StepPlan step_plan(int nx, int ny, int nz, bool xper, int sms, int mode) {
+    StepPlan best{BIGW, 1, nz, 0};
+    double least = 1e300;
+    const long long tx = (xper && nx <= 32) ? 1 : (nx + LXV - 1) / LXV;
+    constexpr double extra = 3.0;
+    for (int w : {BIGW, SMALLW}) {
+        const int th = even_rows(ny, w - 2), bps = BIGW / w;
+        const long long ty = (ny + th - 1) / th, slots = (long long)bps * sms;
+        auto plane = [&](long long blocks) { return w == BIGW ? 2.0 : blocks <= sms ? 1.25 : 1.72; };
+        for (int nc = 1; nc <= nz; ++nc) {
+            const int zc = (nz + nc - 1) / nc;
+            const long long blocks = tx * ty * ((nz + zc - 1) / zc);
+            const double tail = mode == TSLB_MODE_PHASEFIELD ? 3.0 * zc : 0.0;
+            const double cost = (double)((blocks + slots - 1) / slots) * (zc + extra) * plane(blocks) + tail;
+            if (cost < least) { least = cost; best = StepPlan{w, th, zc, 0}; }
+            if (nc > 1 && blocks > 16 * slots) break;   // more waves only add planes outside the chunks
         }
-        if (fill >= 0.9) break;
+        const long long parts = std::min(slots / tx, ty * nz);
+        if (mode != TSLB_MODE_PHASEFIELD && parts > 0 && ty * nz < (1LL << 31)) {
+            const double share = (double)(ty * nz) / parts;
+            const double cost = 1.08 * (share + extra * (share / nz + 1.0)) * plane(parts * tx);
+            if (cost < least) { least = cost; best = StepPlan{w, th, 0, (int)(parts * tx)}; }
+        }
     }
-    const int zc = (nz + best - 1) / best;
-    // Phase field: the curvature makes planes with interface nodes slower, so
-    // tile columns crossing droplets take longer; chunks of 16 planes give
-    // several waves of blocks that the scheduler balances (0.591 -> 0.567 ms on
-    // the 384 x 192 x 128 channel).  The uniform colour step is fastest with
-    // the fewest chunks.
-    if (mode == TSLB_MODE_PHASEFIELD) return std::min(zc, std::max(16, (nz + 7) / 8));
-    return zc;
+    return best;
 }
 
 int launch_normals(tslb_ctx* c) {
@@ -850,7 +878,8 @@ int tslb_create(const tslb_params* p, int nx, int ny, int nz, tslb_ctx** out) {
     if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return bail(e, "cudaStreamSynchronize");
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    c->zchunk = choose_zchunk(step_tiles(nx, ny), nz, sms, kStepBlocksPerSM, p->mode);
+    const StepPlan plan = step_plan(nx, ny, nz, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
+    c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
     if ((e = launch_step_kernel(make_args(c, c->state[0], c->state[1]), p->mode, p->precision, c->stream, false)) != cudaSuccess)
         return bail(e, "cudaFuncSetAttribute");
     *out = c;
@@ -1424,7 +1453,7 @@ int noalloc_fail(int code, const std::string& msg) {
 
 // Once per device, with that device current: resolve the scratch address
 // and set the shared-memory attribute of every step kernel the entry point
-// can launch (FP32 storage, the three modes, x aligned to 16 bytes or not),
+// can launch (FP32 storage, the three modes),
 // so later calls make no first-use runtime calls of their own.
 int noalloc_setup(int dev, NoallocScratch** out) {
     std::lock_guard<std::mutex> lock(g_noalloc_mu);
@@ -1434,13 +1463,14 @@ int noalloc_setup(int dev, NoallocScratch** out) {
         if (e != cudaSuccess) return noalloc_fail(TSLB_ERR_CUDA, std::string("cudaGetSymbolAddress(flags): ") + cudaGetErrorString(e));
         const int modes[3] = {TSLB_MODE_PHASEFIELD, TSLB_MODE_COLOUR, TSLB_MODE_SINGLE};
         for (int mode : modes) {
-            for (int nx : {4, 3}) {   // 16-byte aligned rows, and not
-                StepArgs a;
-                std::memset(&a, 0, sizeof(a));
-                a.nx = nx; a.ny = 1; a.nz = 1; a.zchunk = 1;
-                e = launch_step_kernel(a, mode, TSLB_PREC_FP32, nullptr, false);
-                if (e != cudaSuccess) return noalloc_fail(TSLB_ERR_CUDA, std::string("step kernel attribute: ") + cudaGetErrorString(e));
+            StepArgs a;
+            std::memset(&a, 0, sizeof(a));
+            a.nx = a.ny = a.nz = a.zchunk = a.th = 1;
+            for (int w : {BIGW, SMALLW}) {
+                a.warps = w;
+                if (e == cudaSuccess) e = launch_step_kernel(a, mode, TSLB_PREC_FP32, nullptr, false);
             }
+            if (e != cudaSuccess) return noalloc_fail(TSLB_ERR_CUDA, std::string("step kernel attribute: ") + cudaGetErrorString(e));
         }
         s.ready = true;
     }
@@ -1494,9 +1524,8 @@ extern "C" int tslb_step_noalloc(const tslb_params* p, int nx, int ny, int nz, c
     for (int f = 0; f < NF; ++f) view.scale[f] = 1.0f;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long tiles = step_tiles(nx, ny);
-    const long long want = 4LL * kStepBlocksPerSM * sms;
-    view.zchunk = (int)std::min<long long>(nz, std::max<long long>(8, (tiles * nz + want - 1) / want));
+    const StepPlan plan = step_plan(nx, ny, nz, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
+    view.warps = plan.warps; view.th = plan.th; view.zchunk = plan.zchunk; view.grid = plan.grid;
     StepArgs a = make_args(&view, d_in, d_out);
     if ((e = launch_step_kernel(a, p->mode, TSLB_PREC_FP32, st)) != cudaSuccess)
         return noalloc_fail(TSLB_ERR_CUDA, std::string("step kernel attribute: ") + cudaGetErrorString(e));
@@ -1642,7 +1671,8 @@ int tslb_create_slab(const tslb_params* p, int nx, int ny, int nz, int z_begin, 
     c->zt1 = lo + (z_end - z_begin);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    c->zchunk = choose_zchunk(step_tiles(nx, ny), z_end - z_begin, sms, kStepBlocksPerSM, p->mode);
+    const StepPlan plan = step_plan(nx, ny, z_end - z_begin, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
+    c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
     *out = c;
     return TSLB_OK;
 }
@@ -1674,7 +1704,6 @@ constexpr int kEnsStepWords = 4;   // the ensemble kernel's step counter, ticket
 struct tslb_ensemble {
     std::vector<tslb_ctx*> m;          // member lattices (own state, own params)
     int mode = 0, precision = 0;
-    bool vec = true;
     cudaStream_t stream = nullptr;
     StepArgs* d_args[2] = {nullptr, nullptr};  // per step parity: member args
     WorkItem* d_work = nullptr;
@@ -1720,7 +1749,9 @@ int ens_build(tslb_ensemble* e) {
     for (size_t d = 0; d < e->m.size(); ++d) {
         tslb_ctx* c = e->m[d];
         c->zchunk = std::min(e->zchunk, c->nz);
-        const int gx = (c->nx + TX - 1) / TX, gy = (c->ny + TY - 1) / TY, gz = (c->nz + c->zchunk - 1) / c->zchunk;
+        c->th = even_rows(c->ny, SMALLW - 2);
+        const StepArgs ca = make_args(c, nullptr, nullptr);
+        const int gx = tslb_launch::tiles_x(ca), gy = tslb_launch::tiles_y(ca), gz = (c->nz + c->zchunk - 1) / c->zchunk;
         for (int bz = 0; bz < gz; ++bz)
             for (int by = 0; by < gy; ++by)
                 for (int bx = 0; bx < gx; ++bx) work.push_back(WorkItem{(int)d, bx, by, bz});
@@ -1761,7 +1792,7 @@ int ens_build(tslb_ensemble* e) {
 cudaError_t ens_kernel(tslb_ensemble* e, bool launch) {
     const int grid = e->grid > 0 ? std::min(e->grid, e->nwork) : e->nwork;
     const StepArgs* args = e->d_args[e->parity];
-    return tslb_launch::scalar_ensemble(args, e->d_work, e->nwork, grid, e->mode, e->precision, e->vec, e->d_step,
+    return tslb_launch::scalar_ensemble(args, e->d_work, e->nwork, grid, e->mode, e->precision, e->d_step,
                                         e->stream, launch);
 }
 
@@ -1819,8 +1850,6 @@ int tslb_ensemble_create(const tslb_params* params, const int* dims, int n, tslb
             return efail(nullptr, rc, msg);
         }
         e->m.push_back(c);
-        const int epc = 16 / storage_bytes(e->precision);
-        if (dims[3 * i] % epc) e->vec = false;
     }
     cudaError_t ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
     // step counter of the stochastic rounding (members start at step 0) and launch ticket
@@ -1835,7 +1864,7 @@ int tslb_ensemble_create(const tslb_params* params, const int* dims, int n, tslb
         tslb_ensemble_destroy(e);
         return efail(nullptr, TSLB_ERR_CUDA, msg);
     }
-    e->grid = kStepBlocksPerSM * e->sms;  // persistent: the resident blocks walk the work list
+    e->grid = kEnsBlocksPerSM * e->sms;  // persistent: the resident blocks walk the work list
     int rc = ens_build(e);
     if (rc) {
         std::string msg = e->err;
@@ -1962,7 +1991,7 @@ int tslb_ensemble_tune(tslb_ensemble* e, int* zchunk_out, int* grid_out) {
     // the persistent kernel: two or one resident blocks per SM taking the work
     // items as they finish (one block per item, grid 0, is a tslb_ensemble_set_launch choice)
     const int zcands[] = {8, 16, 32, 64, 128, 1 << 20};
-    const int gcands[] = {kStepBlocksPerSM * e->sms, e->sms};
+    const int gcands[] = {kEnsBlocksPerSM * e->sms, e->sms};
     float best = 1e30f;
     int bz = e->zchunk, bg = e->grid;
     cudaEvent_t t0, t1;

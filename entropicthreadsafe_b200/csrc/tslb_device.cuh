@@ -32,33 +32,17 @@ namespace tslb {
 constexpr int NF = 11;
 enum { F_D = 0, F_U, F_V, F_W, F_XX, F_XY, F_XZ, F_YY, F_YZ, F_ZZ, F_PHI };
 
-// Coefficient slots (per node, shared memory), in five quads and one pair
-// that the pull reads whole, so a source reads a quad with one 16-byte load:
-//   q0 (0, z | zz, c0)        every source
-//   q1 (x, xx | xz, xxz)      sources with cx != 0
-//   q2 (y, yy | yz, yyz)      sources with cy != 0
-//   q3 (xzz, c1 | yzz, c2)    the first half for cx != 0, the second for cy != 0
-//   q4 (xy, xyz | xxy, xyy)   sources with cx != 0 and cy != 0
-//   p5 (c3, c4)               every source (c4: the rest population's)
-// Colour slots c0..c4: phi, Bx, By, Bz, delta0 | phase field: G0, G1x, G1y, G1z, -.
+// Coefficient slots of a node: the 17 monomials of P' and the colour terms
+// c0..c4: phi, Bx, By, Bz, delta0 | phase field: G0, G1x, G1y, G1z, -.
 enum {
-    K_0 = 0, K_Z, K_ZZ, K_C0,
-    K_X, K_XX, K_XZ, K_XXZ,
-    K_Y, K_YY, K_YZ, K_YYZ,
-    K_XZZ, K_C1, K_YZZ, K_C2,
-    K_XY, K_XYZ, K_XXY, K_XYY,
-    K_C3, K_C4,
+    K_0 = 0, K_X, K_Y, K_Z, K_XX, K_YY, K_ZZ, K_XY, K_XZ, K_YZ,
+    K_XXY, K_XXZ, K_XYY, K_YYZ, K_XZZ, K_YZZ, K_XYZ,
+    K_C0, K_C1, K_C2, K_C3, K_C4,
     NCOEF
 };
-constexpr int NQUAD = 5;   // quads q0..q4; slots 4 NQUAD.. form the pair p5
-static_assert(NCOEF == 4 * NQUAD + 2, "coefficient slots: five quads and one pair");
 
 // accumulator slots of a target node
 enum { A_RHO = 0, A_JX, A_JY, A_JZ, A_XX, A_XY, A_XZ, A_YY, A_YZ, A_ZZ, A_COL, NACC };
-
-constexpr int TX = 32;  // block tile in x (one warp row)
-constexpr int TY = 8;   // block tile in y
-constexpr int CW = TX + 2, CH = TY + 2, CAREA = CW * CH;
 
 // lattice weights by |c|^2 (recursive_2c_TSLB3D.f90:71-74)
 __host__ __device__ constexpr float wclass(int c2) {
@@ -78,13 +62,21 @@ struct FaceBC {
 
 struct StepArgs {
     int nx, ny, nz;
+    unsigned plane;         // nx ny
     long long N;            // field stride (elements)
     const void* in;         // 11 fields of the storage type
     void* out;              // 11 fields of the storage type
     float scale[NF];        // stored = value * scale (fp16 storage; 1 otherwise)
     float iscale[NF];       // value = stored * iscale
+    const void* fi[NF];     // the fields of `in` and `out`
+    void* fo[NF];
     const float* nrm;       // phase field: interface normals (3 fields of stride N)
-    int zchunk;             // target planes per block
+    int zchunk;             // target planes per block; 0: `grid` blocks share the tiles' planes equally
+    int grid;
+    int warps;              // warps of a block (tslb_step.cuh: BIGW, SMALLW)
+    int th;                 // target rows of a tile, at most warps - 2
+    int xwrap;              // a warp holds the whole periodic x axis (nx <= 32)
+    int phi_mirror;         // ghost phi is the nearest node's on every face that is not periodic
     int mode;
     float omega_pf;         // 1/tau (phase field)
     float inv_nu_a, inv_nu_b;  // colour: 1/nu of each component
@@ -165,6 +157,7 @@ __device__ __forceinline__ long long nidx(const StepArgs& a, int x, int y, int z
 }
 // periodic wrap of any coordinate into [0, n) (tiles may reach several periods out on tiny lattices)
 __device__ __forceinline__ int wrapi(int c, int n) {
+    if ((unsigned)c < (unsigned)n) return c;
     c %= n;
     return c < 0 ? c + n : c;
 }
@@ -236,12 +229,12 @@ __device__ __forceinline__ unsigned int sr_field(unsigned int hnode, int f) {
     unsigned int h = (hnode + (unsigned int)f * 0x9E3779B9u) * 0x85EBCA6Bu;
     return h ^ (h >> 16);
 }
-// Store fields f and g (g == f: f alone) of one node in 16-bit storage with
+// Store fields f and g (g == f: f alone) of node id in 16-bit storage with
 // one paired conversion: cvt.rn / cvt.rs (stochastic, random bits r) to
 // f16x2 or bf16x2 of the stored values (fp16: value * per-field scale).
 // Returns the largest stored magnitude before rounding, for the range check.
 template <class T>
-__device__ __forceinline__ float store_pair16(T* po, const StepArgs& a, int f, int g, float vf, float vg, int sr,
+__device__ __forceinline__ float store_pair16(const StepArgs& a, unsigned int id, int f, int g, float vf, float vg, int sr,
                                               unsigned int r) {
     constexpr bool H = std::is_same<T, __half>::value;
     const float xf = H ? vf * a.scale[f] : vf, xg = H ? vg * a.scale[g] : vg;
@@ -254,8 +247,8 @@ __device__ __forceinline__ float store_pair16(T* po, const StepArgs& a, int f, i
         else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(xg), "f"(xf));
     }
     // the low half holds field f, the high half field g
-    po[f * a.N] = bits_as<T>((unsigned short)(d & 0xFFFFu));
-    if (g != f) po[g * a.N] = bits_as<T>((unsigned short)(d >> 16));
+    static_cast<T*>(a.fo[f])[id] = bits_as<T>((unsigned short)(d & 0xFFFFu));
+    if (g != f) static_cast<T*>(a.fo[g])[id] = bits_as<T>((unsigned short)(d >> 16));
     return fmaxf(fabsf(xf), fabsf(xg));
 }
 
@@ -316,14 +309,13 @@ __device__ void grad_phi(const StepArgs& a, int x, int y, int z, float g[3]) {
     g[2] = 3.f * gz;
 }
 
-// Arithmetic of the coefficient phase, one operation at a time.  The step
-// computes a node's coefficients in every tile whose coefficient tile holds
-// it: as an own node of one tile and as a rim node of its neighbours.  The
-// populations it sends into different tiles must be the same numbers, or
-// mass is not conserved exactly, so no operation is left for the compiler
-// to contract: Ar1 evaluates one node in FP32, Ar2 two nodes at once on the
-// paired FP32 instructions of sm_100 (one node per lane), and both round
-// every operation identically, lane by lane.
+// Arithmetic of the step, one operation at a time.  The step computes a
+// node's coefficients in every tile that holds it, as a target node of one
+// tile and as a source on the rim of its neighbours.  The populations it
+// sends into different tiles must be the same numbers, or mass is not
+// conserved exactly, so no operation is left for the compiler to contract:
+// Ar1 evaluates one number in FP32, Ar2 two at once on the paired FP32
+// instructions of sm_100.
 struct Ar1 {
     using V = float;
     static __device__ __forceinline__ V c(float x) { return x; }
@@ -341,8 +333,7 @@ struct Ar2 {
     using V = float2;
     static __device__ __forceinline__ V c(float x) { return make_float2(x, x); }
     static __device__ __forceinline__ V add(V x, V y) { return __fadd2_rn(x, y); }
-    // x - y rounded once: fma(y, -1, x)
-    static __device__ __forceinline__ V sub(V x, V y) { return __ffma2_rn(y, make_float2(-1.f, -1.f), x); }
+    static __device__ __forceinline__ V sub(V x, V y) { return __fadd2_rn(x, make_float2(-y.x, -y.y)); }
     static __device__ __forceinline__ V mul(V x, V y) { return __fmul2_rn(x, y); }
     static __device__ __forceinline__ V fma(V x, V y, V z) { return __ffma2_rn(x, y, z); }
     template <class F>
@@ -351,135 +342,143 @@ struct Ar2 {
     static __device__ __forceinline__ V map2(V x, V y, F f) { return make_float2(f(x.x, y.x), f(x.y, y.y)); }
 };
 
-// Per-node coefficients of P'(c) = f_c / w_c - 1 and the colour terms, for
-// one node (Ar1) or two (Ar2).  m[] are the node's 11 moments (m[F_D] =
-// rho - 1).  gphi: colour mode, the gradient of phi; phase field, the
-// interface normal n, with curv the curvature -div n where the interface
-// indicator exceeds 0.2 (else 0).  TAU: the node's relaxation time is
-// tau(phi) + dt (a local eddy-viscosity correction); the surface-tension
-// coefficient follows the corrected omega.
-template <int MODE, bool TAU, class Ar>
-__device__ __forceinline__ void node_coefs_v(const StepArgs& a, const typename Ar::V* m, const typename Ar::V* gphi,
-                                             typename Ar::V curv, typename Ar::V dt, typename Ar::V* K) {
-    using V = typename Ar::V;
-    auto c = [](float x) { return Ar::c(x); };
-    const V d = m[F_D], rho = Ar::add(c(1.f), d);
-    const V u = m[F_U], v = m[F_V], w = m[F_W];
-    const V pxx = m[F_XX], pxy = m[F_XY], pxz = m[F_XZ], pyy = m[F_YY], pyz = m[F_YZ], pzz = m[F_ZZ];
-    const V phi = m[F_PHI];
-    V omega, U, W_, Vv, A = c(0.f), mg = c(0.f), nx_ = c(0.f), ny_ = c(0.f), nz_ = c(0.f);
-    if (MODE == TSLB_MODE_COLOUR) {
-        const V g0 = gphi[0], g1 = gphi[1], g2 = gphi[2];
-        const V m2 = Ar::fma(g2, g2, Ar::fma(g1, g1, Ar::mul(g0, g0)));
-        const float thr2 = a.thr * a.thr;
-        const V rs = Ar::map(m2, [](float x) { return rsqrtf(x); });
-        // branch-free: outside the interface (|g|^2 <= thr^2) A = 0 and n = 0
-        mg = Ar::map2(m2, rs, [thr2](float x, float r) { return x > thr2 ? __fmul_rn(x, r) : 0.f; });
-        const V inv = Ar::map2(m2, rs, [thr2](float x, float r) { return x > thr2 ? r : 0.f; });
-        // 1/nu = (rhoA/rho)/nu_a + (rhoB/rho)/nu_b ; omega = 2/(6 nu + 1) = 2q/(6 + q)
-        const float qa = 0.5f * (a.inv_nu_a + a.inv_nu_b), qd = 0.5f * (a.inv_nu_a - a.inv_nu_b);
-        const V q = Ar::fma(phi, c(qd), c(qa));
-        const V q2 = Ar::add(q, q);
-        // TAU: 1/omega = (6 + q)/(2q) + dtau
-        const V den = TAU ? Ar::fma(q2, dt, Ar::add(q, c(6.f))) : Ar::add(q, c(6.f));
-        omega = Ar::map2(q2, den, [](float n, float e) { return __fdividef(n, e); });
-        nx_ = Ar::mul(g0, inv); ny_ = Ar::mul(g1, inv); nz_ = Ar::mul(g2, inv);
-        const float acs = a.acoef * a.sigma;
-        A = Ar::map2(m2, omega, [thr2, acs](float x, float o) { return x > thr2 ? __fmul_rn(acs, o) : 0.f; });
-        U = u; Vv = v; W_ = w;
-    } else if (MODE == TSLB_MODE_SINGLE) {
-        // fused_TSLB_force_1c: equilibrium at the shifted velocity u + F
-        omega = c(a.omega_pf);
-        U = Ar::add(u, c(a.force[0]));
-        Vv = Ar::add(v, c(a.force[1]));
-        W_ = Ar::add(w, c(a.force[2]));
-    } else {
-        // CSF velocity shift u + sigma kappa n (+ F) (recursive_2c_TSLB3D.f90:630-636,
-        // lb_kernels_module.f90:769)
-        omega = c(a.omega_pf);
-        const V sk = Ar::mul(c(a.sigma), curv);
-        U = Ar::add(Ar::fma(sk, gphi[0], u), c(a.force[0]));
-        Vv = Ar::add(Ar::fma(sk, gphi[1], v), c(a.force[1]));
-        W_ = Ar::add(Ar::fma(sk, gphi[2], w), c(a.force[2]));
-        nx_ = gphi[0]; ny_ = gphi[1]; nz_ = gphi[2];
-    }
-    const V om1 = Ar::sub(c(1.f), omega);
-    // recursive third-order non-equilibrium moments a3 = u_a Pi_bc + perms
-    const V u2 = Ar::add(u, u), v2 = Ar::add(v, v), w2 = Ar::add(w, w);
-    const V a_xxy = Ar::fma(v, pxx, Ar::mul(u2, pxy));
-    const V a_xxz = Ar::fma(w, pxx, Ar::mul(u2, pxz));
-    const V a_xyy = Ar::fma(v2, pxy, Ar::mul(u, pyy));
-    const V a_yyz = Ar::fma(w, pyy, Ar::mul(v2, pyz));
-    const V a_xzz = Ar::fma(w2, pxz, Ar::mul(u, pzz));
-    const V a_yzz = Ar::fma(w2, pyz, Ar::mul(v, pzz));
-    const V a_xyz = Ar::fma(w, pxy, Ar::fma(v, pxz, Ar::mul(u, pyz)));
-    const V rU = Ar::mul(rho, U), rV = Ar::mul(rho, Vv), rW = Ar::mul(rho, W_);
-    // second-order equilibrium products rho U_a U_b
-    const V rUU = Ar::mul(rU, U), rVV = Ar::mul(rV, Vv), rWW = Ar::mul(rW, W_);
-    const V rUV = Ar::mul(rU, Vv), rUW = Ar::mul(rU, W_), rVW = Ar::mul(rV, W_);
-    // full third-order coefficients: rho U_a U_b U_c + (1 - omega) a3
-    const V t_xxy = Ar::fma(om1, a_xxy, Ar::mul(rUU, Vv)), t_xxz = Ar::fma(om1, a_xxz, Ar::mul(rUU, W_));
-    const V t_xyy = Ar::fma(om1, a_xyy, Ar::mul(rUV, Vv)), t_yyz = Ar::fma(om1, a_yyz, Ar::mul(rVV, W_));
-    const V t_xzz = Ar::fma(om1, a_xzz, Ar::mul(rUW, W_)), t_yzz = Ar::fma(om1, a_yzz, Ar::mul(rVW, W_));
-    const V t_xyz = Ar::fma(om1, a_xyz, Ar::mul(rUV, W_));
-    const V tr = Ar::add(Ar::add(pxx, pyy), pzz);
-    // K0 = d - 1.5 (rho |U|^2 + (1 - omega) tr Pi)
-    K[K_0] = Ar::fma(Ar::mul(c(-1.5f), om1), tr, Ar::fma(c(-1.5f), Ar::add(Ar::add(rUU, rVV), rWW), d));
-    K[K_X] = Ar::fma(c(-4.5f), Ar::add(t_xyy, t_xzz), Ar::mul(c(3.f), rU));
-    K[K_Y] = Ar::fma(c(-4.5f), Ar::add(t_xxy, t_yzz), Ar::mul(c(3.f), rV));
-    K[K_Z] = Ar::fma(c(-4.5f), Ar::add(t_xxz, t_yyz), Ar::mul(c(3.f), rW));
-    K[K_XX] = Ar::mul(c(4.5f), Ar::fma(om1, pxx, rUU));
-    K[K_YY] = Ar::mul(c(4.5f), Ar::fma(om1, pyy, rVV));
-    K[K_ZZ] = Ar::mul(c(4.5f), Ar::fma(om1, pzz, rWW));
-    K[K_XY] = Ar::mul(c(9.f), Ar::fma(om1, pxy, rUV));
-    K[K_XZ] = Ar::mul(c(9.f), Ar::fma(om1, pxz, rUW));
-    K[K_YZ] = Ar::mul(c(9.f), Ar::fma(om1, pyz, rVW));
-    K[K_XXY] = Ar::mul(c(13.5f), t_xxy);
-    K[K_XXZ] = Ar::mul(c(13.5f), t_xxz);
-    K[K_XYY] = Ar::mul(c(13.5f), t_xyy);
-    K[K_YYZ] = Ar::mul(c(13.5f), t_yyz);
-    K[K_XZZ] = Ar::mul(c(13.5f), t_xzz);
-    K[K_YZZ] = Ar::mul(c(13.5f), t_yzz);
-    K[K_XYZ] = Ar::mul(c(27.f), t_xyz);
-    if (MODE == TSLB_MODE_COLOUR) {
-        // force as population source 3 w c.F (recursive_colorTSLB3D.f90:776)
-        K[K_X] = Ar::add(K[K_X], c(3.f * a.force[0]));
-        K[K_Y] = Ar::add(K[K_Y], c(3.f * a.force[1]));
-        K[K_Z] = Ar::add(K[K_Z], c(3.f * a.force[2]));
-        // perturbation (A/2)|g| [w (c.n)^2 - B_i], B_i = w_i for i >= 1 (A = 0 off the interface)
-        const V h = Ar::mul(Ar::mul(c(0.5f), A), mg), h2 = Ar::add(h, h);
-        K[K_0] = Ar::sub(K[K_0], h);
-        K[K_XX] = Ar::fma(Ar::mul(h, nx_), nx_, K[K_XX]);
-        K[K_YY] = Ar::fma(Ar::mul(h, ny_), ny_, K[K_YY]);
-        K[K_ZZ] = Ar::fma(Ar::mul(h, nz_), nz_, K[K_ZZ]);
-        K[K_XY] = Ar::fma(Ar::mul(h2, nx_), ny_, K[K_XY]);
-        K[K_XZ] = Ar::fma(Ar::mul(h2, nx_), nz_, K[K_XZ]);
-        K[K_YZ] = Ar::fma(Ar::mul(h2, ny_), nz_, K[K_YZ]);
+// Coefficients of P'(c) = f_c / w_c - 1 of a node.  With r = 4.5 rho
+// and o = 4.5 (1 - omega) the second-order coefficients are
+//   K_ab = (2 - delta_ab) (r u_a u_b + o Pi_ab),
+// and the third-order ones, 13.5 (rho u_a u_a u_b + (1 - omega) a3_aab) with
+// the recursive a3_aab = u_b Pi_aa + 2 u_a Pi_ab, come from them:
+//   K_aab = 3 u_b K_aa + 3 u_a (2 o Pi_ab).
+// m[] are the node's moments (m[F_D] = rho - 1).
+
+// Colour mode: g is the gradient of phi, m[F_PHI] phi; TAU: the relaxation
+// time is tau(phi) + dt (a local eddy-viscosity correction; the
+// surface-tension coefficient follows the corrected omega).  Returns whether
+// any node of the warp lies on the interface; if none does, the recolouring
+// terms K_C1..K_C3 are 0 in the whole warp.
+template <bool TAU>
+__device__ __forceinline__ bool coefs_colour(const StepArgs& a, const float* m, const float* g, float dt, float* K) {
+    using A = Ar1;
+    using V = A::V;
+    auto c = [](float x) { return A::c(x); };
+    const V d = m[F_D], u = m[F_U], v = m[F_V], w = m[F_W], phi = m[F_PHI];
+    // 1/nu = (rhoA/rho)/nu_a + (rhoB/rho)/nu_b ; omega = 2/(6 nu + 1) = 2q/(6 + q)
+    const float qa = 0.5f * (a.inv_nu_a + a.inv_nu_b), qd = 0.5f * (a.inv_nu_a - a.inv_nu_b);
+    const V q = A::fma(phi, c(qd), c(qa)), q2 = A::add(q, q);
+    // TAU: 1/omega = (6 + q)/(2q) + dtau
+    const V den = TAU ? A::fma(q2, dt, A::add(q, c(6.f))) : A::add(q, c(6.f));
+    const V omega = A::map2(q2, den, [](float n, float e) { return __fdividef(n, e); });
+    const V rho = A::add(c(1.f), d), om1 = A::sub(c(1.f), omega);
+    const V o = A::mul(om1, c(4.5f)), o2 = A::add(o, o), r = A::mul(rho, c(4.5f));
+    const V ru = A::mul(r, u), rv = A::mul(r, v), rw = A::mul(r, w), ru2 = A::add(ru, ru), rv2 = A::add(rv, rv);
+    const V xx = A::fma(o, m[F_XX], A::mul(ru, u)), yy = A::fma(o, m[F_YY], A::mul(rv, v)), zz = A::fma(o, m[F_ZZ], A::mul(rw, w));
+    const V pxy = A::mul(o2, m[F_XY]), pxz = A::mul(o2, m[F_XZ]), pyz = A::mul(o2, m[F_YZ]);
+    const V xy = A::fma(ru2, v, pxy), xz = A::fma(ru2, w, pxz), yz = A::fma(rv2, w, pyz);
+    const V u3 = A::mul(u, c(3.f)), v3 = A::mul(v, c(3.f)), w3 = A::mul(w, c(3.f));
+    K[K_XXY] = A::fma(v3, xx, A::mul(u3, pxy));
+    K[K_XXZ] = A::fma(w3, xx, A::mul(u3, pxz));
+    K[K_XYY] = A::fma(u3, yy, A::mul(v3, pxy));
+    K[K_YYZ] = A::fma(w3, yy, A::mul(v3, pyz));
+    K[K_XZZ] = A::fma(u3, zz, A::mul(w3, pxz));
+    K[K_YZZ] = A::fma(v3, zz, A::mul(w3, pyz));
+    K[K_XYZ] = A::fma(u3, yz, A::fma(v3, pxz, A::mul(w3, pxy)));
+    // K_a = 3 rho u_a - (K_abb + K_acc)/3, with the force as population source
+    // 3 w c.F (recursive_colorTSLB3D.f90:776)
+    const V mt = c(-1.f / 3.f), tt = c(2.f / 3.f);
+    K[K_X] = A::fma(mt, A::add(K[K_XYY], K[K_XZZ]), A::fma(tt, ru, c(3.f * a.force[0])));
+    K[K_Y] = A::fma(mt, A::add(K[K_XXY], K[K_YZZ]), A::fma(tt, rv, c(3.f * a.force[1])));
+    K[K_Z] = A::fma(mt, A::add(K[K_XXZ], K[K_YYZ]), A::fma(tt, rw, c(3.f * a.force[2])));
+    K[K_0] = A::fma(mt, A::add(A::add(xx, yy), zz), d);
+    K[K_XX] = xx; K[K_YY] = yy; K[K_ZZ] = zz; K[K_XY] = xy; K[K_XZ] = xz; K[K_YZ] = yz;
+    K[K_C0] = phi; K[K_C1] = K[K_C2] = K[K_C3] = K[K_C4] = c(0.f);
+    const V m2 = A::fma(g[2], g[2], A::fma(g[1], g[1], A::mul(g[0], g[0])));
+    const float thr2 = a.thr * a.thr;
+    const bool iface = __any_sync(0xffffffffu, m2 > thr2);
+    if (iface) {
+        const V rs = A::map(m2, [](float x) { return rsqrtf(x); });
+        // outside the interface (|g|^2 <= thr^2) |g| and n are 0
+        const V mg = A::map2(m2, rs, [thr2](float x, float y) { return x > thr2 ? __fmul_rn(x, y) : 0.f; });
+        const V inv = A::map2(m2, rs, [thr2](float x, float y) { return x > thr2 ? y : 0.f; });
+        const V nx = A::mul(g[0], inv), ny = A::mul(g[1], inv), nz = A::mul(g[2], inv);
+        // perturbation (A/2)|g| [w (c.n)^2 - B_i], B_i = w_i for i >= 1
+        const V Am = A::mul(A::mul(c(a.acoef * a.sigma), omega), mg);
+        const V h = A::mul(c(0.5f), Am), h2 = Am;
+        const V hx = A::mul(h, nx), hy = A::mul(h, ny), hz = A::mul(h, nz), hx2 = A::mul(h2, nx), hy2 = A::mul(h2, ny);
+        K[K_0] = A::sub(K[K_0], h);
+        K[K_XX] = A::fma(hx, nx, xx);
+        K[K_YY] = A::fma(hy, ny, yy);
+        K[K_ZZ] = A::fma(hz, nz, zz);
+        K[K_XY] = A::fma(hx2, ny, xy);
+        K[K_XZ] = A::fma(hx2, nz, xz);
+        K[K_YZ] = A::fma(hy2, nz, yz);
         // rest population: B_0 = -10/27 instead of w_0
-        const V d0 = Ar::mul(Ar::mul(A, c(1.f / 3.f)), mg);
-        // recolouring 2 beta (rhoA rhoB / rho) n  (published form, cos theta; n = 0 off the interface)
-        const V bb = Ar::mul(Ar::mul(c(0.5f * a.beta), rho), Ar::fma(Ar::mul(c(-1.f), phi), phi, c(1.f)));
-        K[K_C0] = phi; K[K_C1] = Ar::mul(bb, nx_); K[K_C2] = Ar::mul(bb, ny_); K[K_C3] = Ar::mul(bb, nz_); K[K_C4] = d0;
-    } else if (MODE == TSLB_MODE_SINGLE) {
-        K[K_C0] = c(0.f); K[K_C1] = c(0.f); K[K_C2] = c(0.f); K[K_C3] = c(0.f); K[K_C4] = c(0.f);
-    } else if (MODE == TSLB_MODE_PHASEFIELD) {
-        // D3Q7 phase field: g_q = G0 + e_q.G1 (recursive_2c_TSLB3D.f90:808-831)
-        const V sh = Ar::mul(Ar::mul(c(0.125f * a.sharp), phi), Ar::sub(c(1.f), phi));
-        const V p3 = Ar::mul(c(0.375f), phi);
-        K[K_C0] = Ar::mul(c(0.125f), phi);
-        K[K_C1] = Ar::fma(sh, nx_, Ar::mul(p3, u));
-        K[K_C2] = Ar::fma(sh, ny_, Ar::mul(p3, v));
-        K[K_C3] = Ar::fma(sh, nz_, Ar::mul(p3, w));
-        K[K_C4] = c(0.f);
+        K[K_C4] = A::mul(Am, c(1.f / 3.f));
+        // recolouring 2 beta (rhoA rhoB / rho) n  (published form, cos theta)
+        const V bb = A::mul(A::mul(c(0.5f * a.beta), rho), A::fma(A::mul(c(-1.f), phi), phi, c(1.f)));
+        K[K_C1] = A::mul(bb, nx); K[K_C2] = A::mul(bb, ny); K[K_C3] = A::mul(bb, nz);
     }
+    return iface;
 }
 
-// one node (the call sites of the phase field and of single lattices)
-template <int MODE, bool TAU = false>
-__device__ __forceinline__ void node_coefs(const StepArgs& a, const float* m, const float* gphi, float curv, float* K,
-                                           long long id = 0) {
-    const float dt = TAU ? __ldg(a.dtau + id) : 0.f;
-    node_coefs_v<MODE, TAU, Ar1>(a, m, gphi, curv, dt, K);
+// Coefficients K_0 .. K_XYZ with the equilibrium at (1 + d, U) and the
+// non-equilibrium part of the node's u and Pi: f^eq(1 + d, U) + om1 w a^neq(Pi, u).
+__device__ __forceinline__ void coefs_moments(float d, const float* m, float U, float Vv, float W, float om1, float* K) {
+    using A = Ar1;
+    using V = float;
+    auto c = [](float x) { return A::c(x); };
+    const V u = m[F_U], v = m[F_V], w = m[F_W];
+    const V rho = A::add(c(1.f), d);
+    const V o = A::mul(c(4.5f), om1), o2 = A::add(o, o), r = A::mul(rho, c(4.5f));
+    const V ru = A::mul(r, U), rv = A::mul(r, Vv), rw = A::mul(r, W), ru2 = A::add(ru, ru), rv2 = A::add(rv, rv);
+    // equilibrium (e) and non-equilibrium (p) parts of the second order
+    const V exx = A::mul(ru, U), eyy = A::mul(rv, Vv), ezz = A::mul(rw, W);
+    const V pxx = A::mul(o, m[F_XX]), pyy = A::mul(o, m[F_YY]), pzz = A::mul(o, m[F_ZZ]);
+    const V pxy = A::mul(o2, m[F_XY]), pxz = A::mul(o2, m[F_XZ]), pyz = A::mul(o2, m[F_YZ]);
+    const V eyz = A::mul(rv2, W);
+    K[K_XX] = A::add(exx, pxx); K[K_YY] = A::add(eyy, pyy); K[K_ZZ] = A::add(ezz, pzz);
+    K[K_XY] = A::fma(ru2, Vv, pxy); K[K_XZ] = A::fma(ru2, W, pxz); K[K_YZ] = A::add(eyz, pyz);
+    const V u3 = A::mul(u, c(3.f)), v3 = A::mul(v, c(3.f)), w3 = A::mul(w, c(3.f));
+    const V U3 = A::mul(U, c(3.f)), V3 = A::mul(Vv, c(3.f)), W3 = A::mul(W, c(3.f));
+    K[K_XXY] = A::fma(V3, exx, A::fma(v3, pxx, A::mul(u3, pxy)));
+    K[K_XXZ] = A::fma(W3, exx, A::fma(w3, pxx, A::mul(u3, pxz)));
+    K[K_XYY] = A::fma(U3, eyy, A::fma(u3, pyy, A::mul(v3, pxy)));
+    K[K_YYZ] = A::fma(W3, eyy, A::fma(w3, pyy, A::mul(v3, pyz)));
+    K[K_XZZ] = A::fma(U3, ezz, A::fma(u3, pzz, A::mul(w3, pxz)));
+    K[K_YZZ] = A::fma(V3, ezz, A::fma(v3, pzz, A::mul(w3, pyz)));
+    K[K_XYZ] = A::fma(U3, eyz, A::fma(u3, pyz, A::fma(v3, pxz, A::mul(w3, pxy))));
+    const V mt = c(-1.f / 3.f), tt = c(2.f / 3.f);
+    K[K_X] = A::fma(mt, A::add(K[K_XYY], K[K_XZZ]), A::mul(tt, ru));
+    K[K_Y] = A::fma(mt, A::add(K[K_XXY], K[K_YZZ]), A::mul(tt, rv));
+    K[K_Z] = A::fma(mt, A::add(K[K_XXZ], K[K_YYZ]), A::mul(tt, rw));
+    K[K_0] = A::fma(mt, A::add(A::add(K[K_XX], K[K_YY]), K[K_ZZ]), d);
+}
+
+// Phase field (PHASE: the equilibrium at the CSF-shifted velocity
+// u + sigma kappa n (+ F), recursive_2c_TSLB3D.f90:630-636,
+// lb_kernels_module.f90:769; n the interface normal, curv the curvature
+// -div n where the interface indicator exceeds 0.2, else 0) and single
+// component (fused_TSLB_force_1c: at u + F).
+template <bool PHASE>
+__device__ __forceinline__ void coefs_shifted(const StepArgs& a, const float* m, const float* n, float curv, float* K) {
+    using A = Ar1;
+    using V = float;
+    auto c = [](float x) { return A::c(x); };
+    const V u = m[F_U], v = m[F_V], w = m[F_W];
+    V U = A::add(u, c(a.force[0])), Vv = A::add(v, c(a.force[1])), W = A::add(w, c(a.force[2]));
+    if (PHASE) {
+        const V sk = A::mul(c(a.sigma), curv);
+        U = A::fma(sk, n[0], U); Vv = A::fma(sk, n[1], Vv); W = A::fma(sk, n[2], W);
+    }
+    coefs_moments(m[F_D], m, U, Vv, W, 1.f - a.omega_pf, K);
+    K[K_C0] = K[K_C1] = K[K_C2] = K[K_C3] = K[K_C4] = c(0.f);
+    if (PHASE) {
+        // D3Q7 phase field: g_q = G0 + e_q.G1 (recursive_2c_TSLB3D.f90:808-831)
+        const V phi = m[F_PHI];
+        const V sh = A::mul(A::mul(c(0.125f * a.sharp), phi), A::sub(c(1.f), phi)), p3 = A::mul(c(0.375f), phi);
+        K[K_C0] = A::mul(c(0.125f), phi);
+        K[K_C1] = A::fma(sh, n[0], A::mul(p3, u));
+        K[K_C2] = A::fma(sh, n[1], A::mul(p3, v));
+        K[K_C3] = A::fma(sh, n[2], A::mul(p3, w));
+    }
 }
 
 // P'(c) for a runtime direction (boundary paths)
@@ -495,7 +494,8 @@ __device__ __forceinline__ float eval_P(const float* K, long long stride, int cx
 }
 
 // accumulate population value f (already weighted) of direction c into acc
-__device__ __forceinline__ void acc_dir_rt(float* acc, int cx, int cy, int cz, float f) {
+template <class Acc>
+__device__ __forceinline__ void acc_dir_rt(const Acc& acc, int cx, int cy, int cz, float f) {
     acc[A_RHO] += f;
     acc[A_JX] += cx * f; acc[A_JY] += cy * f; acc[A_JZ] += cz * f;
     acc[A_XX] += (cx * cx) * f; acc[A_YY] += (cy * cy) * f; acc[A_ZZ] += (cz * cz) * f;

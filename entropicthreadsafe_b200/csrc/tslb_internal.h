@@ -35,7 +35,8 @@ struct tslb_ctx {
     int red_queued = 0;
     int red_blocks = 0;
     bool loaded = false;
-    int zchunk = 32;
+    int zchunk = 32, grid = 0;             // target planes per block of the step; 0: `grid` blocks share them
+    int warps = 16, th = 1;    // warps per block and target rows per tile of the step
     // z slab of a larger lattice (tslb_create_slab): the local array holds
     // halo_lo + owned + halo_hi planes; a step updates planes [zt0, zt1)
     int zt0 = 0, zt1 = 0;                  // zt1 = 0: all planes

@@ -1,234 +1,214 @@
 // tslb_step.cuh -- the fused pull step kernel.
 //
-// One CUDA block owns a TX x TY tile of (x, y) columns and a chunk of
-// `zchunk` target planes.  It marches through the source planes
-// s = z0-1 .. z1 of the chunk; for each:
-//   0. the moments of plane s+1 and phi of plane s+2 are copied into shared
-//      memory with cp.async (16-byte chunks when nx % 4 == 0), overlapping
-//      the work on plane s;
-//   1. every thread computes the coefficients of P'(c) (tslb_device.cuh) of
-//      one or two nodes of plane s (the tile plus a one-node rim) into
-//      shared memory (double buffered);
-//   2. every thread pulls, for its own column, the 27 populations that
-//      leave the 9 source nodes (x-ox, y-oy, s) and land on targets
-//      (x, y, s-1), (x, y, s), (x, y, s+1), accumulating the targets'
-//      moments in registers;
-//   3. populations whose source lies behind a non-periodic face are
-//      supplied at the target from its own node (bounce-back, regularized
-//      velocity faces);
-//   4. target plane s-1 is complete: its 11 moments are written out.
-// One CTA barrier per plane, between 1 and 2: before it every thread waits
-// for its own copies of step 0, so the barrier publishes the coefficients of
-// plane s and the staged data of plane s+1 alike.
+// A block owns a tile of (x, y) columns and a chunk of `zchunk` target
+// planes, and marches through the source planes s = z0-1 .. z1 of the chunk.
+// A warp is one row of 32 source nodes, one per thread.  The outermost lanes
+// and rows of a tile are sources only: 30 x (W - 2) targets per block of W
+// warps.
+//
+// The populations that land on a node are never formed one by one.  A
+// post-collision population is f_c = w_c (1 + P'(c)) with P' a polynomial of
+// 17 coefficients in cx, cy, cz, and w_c = w(cx) w(cy) w(cz) is a product, so
+// the moments of the 27 pulled populations,
+//   M_abc(x) = sum_c cx^a cy^b cz^c w_c P'_{x-c}(c),
+// factor into three one-dimensional sums, one axis after the other:
+//   x  every monomial cy^j cz^k of P' is evaluated at cx = -1, 0, 1 and pulled
+//      from the two neighbouring lanes (shuffles), summed with cx^a;
+//   y  the results, polynomials in cy, are evaluated at cy = -1, 0, 1 and
+//      exchanged with the neighbouring warps through shared memory;
+//   z  the results, polynomials in cz, are added to the targets s-1, s, s+1,
+//      whose partial sums stay in registers.
+// Three sums of three terms instead of one of 27: about 265 FP32 operations per
+// node with the coefficients, against about 560 for a pull of the 27
+// populations from a tile of coefficients.
+//
+// Per source plane s:
+//   0. phi of a plane ahead is read for the block's ring of phi planes;
+//   1. every thread forms the coefficients of its node, the x sums and the y
+//      values it sends;
+//   2. one CTA barrier publishes the y values and the phi plane;
+//   3. the moments of plane s+1 are read ahead, the y and z sums completed,
+//      populations whose source lies behind a non-periodic face or in an
+//      interior solid added, and target plane s-1 written out.
 // Reading moments and writing moments is all the HBM traffic there is:
 // the populations f, g of the reference (recursive_2c_TSLB3D.f90:54) never
 // exist in memory.
+//
+// What bounds it: the latency of the chain through a plane, not HBM.  On the
+// 384 x 192 x 128 colour channel (FP32) a step takes 0.35 ms on a B200, where
+// the kernel that pulled 27 populations took 0.45 ms (1109 thread instructions
+// a node, issue active 62%) and 88 B a node at the measured copy rate take
+// 0.129 ms.  A warp spends 572 instructions on a row and plane (640 a target
+// node with the rims), issue is active 58% of the cycles; the stalls are spread
+// over shared-memory and shuffle latency, fixed instruction latency and the
+// plane barrier.  So registers buy more than instructions: 16 warps of 128
+// registers an SM without a spill (a spilled word comes back from L2, as shared
+// memory leaves little L1: 24 bytes of spills in the plane loop cost 12%); two
+// rows a thread on paired FP32 instructions needs 5/7 of the instructions a row
+// but 255 registers, and 8 warps an SM were slower (0.51 ms), 12 with spills
+// slower still (0.66 ms).
 #pragma once
 
 #include "tslb_device.cuh"
 
 namespace tslb {
 
-// Coefficients live in shared memory as NQUAD planes of CAREA float4 and one
-// plane of CAREA float2: node n's quad q is at float offset q * 4 CAREA + 4 n,
-// its pair p5 at PAIR_OFF + 2 n.  A source loads each quad its directions use
-// with one 16-byte load (lanes, consecutive x, read consecutive 16-byte
-// words), or the half of q3 it uses with an 8-byte load.
-constexpr int PAIR_OFF = 4 * NQUAD * CAREA;
-// a node of the coefficient tile: its quad-plane and pair-plane addresses
-struct CNode {
-    const float* q;   // coef + 4 n
-    const float* p;   // coef + PAIR_OFF + 2 n
-    __device__ __forceinline__ CNode at(int dn) const { return CNode{q + 4 * dn, p + 2 * dn}; }
-};
-__device__ __forceinline__ CNode cnode(const float* coef, int n) { return CNode{coef + 4 * n, coef + PAIR_OFF + 2 * n}; }
-__device__ __forceinline__ float comp4(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
-// slot of node c: HALF reads the half of its quad that holds it (8 bytes)
-template <bool HALF = false>
-__device__ __forceinline__ float coef_at(const CNode& c, int slot) {
-    if (slot >= 4 * NQUAD) {
-        const float2 v = *reinterpret_cast<const float2*>(c.p);
-        return slot & 1 ? v.y : v.x;
-    }
-    const float* b = c.q + (slot >> 2) * (4 * CAREA);
-    if (HALF) {
-        const float2 v = *reinterpret_cast<const float2*>(b + (slot & 2));
-        return slot & 1 ? v.y : v.x;
-    }
-    return comp4(*reinterpret_cast<const float4*>(b), slot & 3);
+// Slot of the monomial cx^i cy^j cz^k of P'
+__host__ __device__ constexpr int kslot(int i, int j, int k) {
+    return i + j + k == 0 ? K_0
+         : i + j + k == 1 ? (i ? K_X : j ? K_Y : K_Z)
+         : i + j + k == 2 ? (i == 2 ? K_XX : j == 2 ? K_YY : k == 2 ? K_ZZ : !k ? K_XY : !j ? K_XZ : K_YZ)
+         : i == 1 && j == 1 ? K_XYZ : i == 2 ? (j ? K_XXY : K_XXZ) : j == 2 ? (i ? K_XYY : K_YYZ) : (i ? K_XZZ : K_YZZ);
 }
-// (single-component mode leaves the colour slots unset: stored, never read)
-template <int MODE>
-__device__ __forceinline__ void store_coefs(float* coef, int n, const float* K) {
-#pragma unroll
-    for (int q = 0; q < NQUAD; ++q)
-        *reinterpret_cast<float4*>(coef + q * (4 * CAREA) + 4 * n) = make_float4(K[4 * q], K[4 * q + 1], K[4 * q + 2], K[4 * q + 3]);
-    *reinterpret_cast<float2*>(coef + PAIR_OFF + 2 * n) = make_float2(K[4 * NQUAD], K[4 * NQUAD + 1]);
+// the same with exponents along a face's normal axis AX and the two axes after it (cyclic)
+template <int AX>
+__host__ __device__ constexpr int kslot_ax(int n, int p, int q) {
+    return AX == 0 ? kslot(n, p, q) : AX == 1 ? kslot(q, n, p) : kslot(p, q, n);
 }
-
-// P' = Q0 + cz Q1 + cz^2 Q2 of the directions (CXv, CYv, cz), cz = -1, 0, 1,
-// of the source at coefficient node Kp
-template <int CXv, int CYv>
-struct Src {
-    CNode Kp;
-    // q3 is read whole only by sources that use both of its halves
-    __device__ __forceinline__ float L(int slot) const {
-        return (slot >> 2) == 3 && !(CXv && CYv) ? coef_at<true>(Kp, slot) : coef_at<false>(Kp, slot);
-    }
-    __device__ __forceinline__ void eval(float& Pm, float& P0, float& Pp) const {
-        float q0 = L(K_0);
-        if (CXv) q0 += CXv * L(K_X) + L(K_XX);
-        if (CYv) q0 += CYv * L(K_Y) + L(K_YY);
-        if (CXv && CYv) q0 += (CXv * CYv) * L(K_XY) + CYv * L(K_XXY) + CXv * L(K_XYY);
-        float q1 = L(K_Z);
-        if (CXv) q1 += CXv * L(K_XZ) + L(K_XXZ);
-        if (CYv) q1 += CYv * L(K_YZ) + L(K_YYZ);
-        if (CXv && CYv) q1 += (CXv * CYv) * L(K_XYZ);
-        float q2 = L(K_ZZ);
-        if (CXv) q2 += CXv * L(K_XZZ);
-        if (CYv) q2 += CYv * L(K_YZZ);
-        const float t = q0 + q2;
-        Pm = t - q1;
-        P0 = q0;
-        Pp = t + q1;
-    }
-};
-
-// The mirror sources of cx = +1 and cx = -1 (same cy) evaluated together as
-// one float2 on the paired FP32 instructions of sm_100 (x: cx = +1, y: cx = -1);
-// the factors +-1 are exact, so each lane is the scalar evaluation.
-template <int CYv>
-struct SrcPair {
-    Src<1, CYv> A;    // source of cx = +1
-    Src<-1, CYv> B;   // source of cx = -1
-    __device__ __forceinline__ float2 L(int slot) const { return make_float2(A.L(slot), B.L(slot)); }
-    __device__ __forceinline__ void eval(float2& Pm, float2& P0, float2& Pp) const {
-        const float2 sx = make_float2(1.f, -1.f);
-        float2 q0 = __fadd2_rn(L(K_0), __ffma2_rn(sx, L(K_X), L(K_XX)));
-        float2 q1 = __fadd2_rn(L(K_Z), __ffma2_rn(sx, L(K_XZ), L(K_XXZ)));
-        float2 q2 = __ffma2_rn(sx, L(K_XZZ), L(K_ZZ));
-        if (CYv) {
-            const float2 cy = make_float2((float)CYv, (float)CYv), sxy = make_float2((float)CYv, (float)-CYv);
-            q0 = __fadd2_rn(q0, __ffma2_rn(cy, L(K_Y), L(K_YY)));
-            q0 = __fadd2_rn(q0, __ffma2_rn(sxy, L(K_XY), __ffma2_rn(cy, L(K_XXY), __fmul2_rn(sx, L(K_XYY)))));
-            q1 = __fadd2_rn(q1, __ffma2_rn(cy, L(K_YZ), L(K_YYZ)));
-            q1 = __ffma2_rn(sxy, L(K_XYZ), q1);
-            q2 = __ffma2_rn(cy, L(K_YZZ), q2);
-        }
-        const float2 t = __fadd2_rn(q0, q2);
-        Pm = __ffma2_rn(make_float2(-1.f, -1.f), q1, t);
-        P0 = q0;
-        Pp = __fadd2_rn(t, q1);
-    }
-};
-
-__host__ __device__ constexpr float w1d(int c) { return c == 0 ? 2.0f / 3.0f : 1.0f / 6.0f; }
-
-// Moments of the three populations of one (cy, cz) group: directions
-// (+1, cy, cz), (0, cy, cz), (-1, cy, cz) with values a, c0, b (unweighted
-// P'), folded through S = a + b, D = a - b and T = S + (wC/wE) c0, each
-// accumulated with the weight wE of the x-moving directions (wC/wE = 4).
-template <int CYv, int CZv>
-__device__ __forceinline__ void acc_group(float* acc, float a, float c0, float b) {
-    constexpr float wE = w1d(1) * w1d(CYv) * w1d(CZv);
-    constexpr float pe = wE, ne = -wE;
-    const float S = a + b, D = a - b, T = fmaf(w1d(0) / w1d(1), c0, S);
-    acc[A_RHO] = fmaf(pe, T, acc[A_RHO]);
-    acc[A_JX] = fmaf(pe, D, acc[A_JX]);
-    acc[A_XX] = fmaf(pe, S, acc[A_XX]);
-    if (CYv) {
-        acc[A_JY] = fmaf(CYv > 0 ? pe : ne, T, acc[A_JY]);
-        acc[A_YY] = fmaf(pe, T, acc[A_YY]);
-        acc[A_XY] = fmaf(CYv > 0 ? pe : ne, D, acc[A_XY]);
-    }
-    if (CZv) {
-        acc[A_JZ] = fmaf(CZv > 0 ? pe : ne, T, acc[A_JZ]);
-        acc[A_ZZ] = fmaf(pe, T, acc[A_ZZ]);
-        acc[A_XZ] = fmaf(CZv > 0 ? pe : ne, D, acc[A_XZ]);
-    }
-    if (CYv && CZv) acc[A_YZ] = fmaf(CYv * CZv > 0 ? pe : ne, T, acc[A_YZ]);
+__host__ __device__ constexpr int aslot(int p, int q) {   // second-order accumulator of axes p, q
+    return p == q ? (p == 0 ? A_XX : p == 1 ? A_YY : A_ZZ) : p + q == 1 ? A_XY : p + q == 2 ? A_XZ : A_YZ;
+}
+// Moments of the nine populations w_c P(r c) with c = s along the normal axis
+// AX (s, r = +-1): P is a polynomial and the weights are products, so the sums
+// over the two other axes are closed (sum w = 1, sum w c^2 = sum w c^4 = 1/3).
+template <int AX, class Acc>
+__device__ __forceinline__ void face_sum(const float* K, float s, float r, const Acc& acc) {
+    constexpr int P = (AX + 1) % 3, Q = (AX + 2) % 3;
+    constexpr float t = 1.f / 3.f;
+    auto k = [&](int n, int p, int q) { return K[kslot_ax<AX>(n, p, q)]; };
+    const float rs = r * s;
+    const float q00 = k(0, 0, 0) + k(2, 0, 0) + rs * k(1, 0, 0);
+    const float q10 = r * (k(0, 1, 0) + k(2, 1, 0)) + s * k(1, 1, 0), q01 = r * (k(0, 0, 1) + k(2, 0, 1)) + s * k(1, 0, 1);
+    const float q20 = k(0, 2, 0) + rs * k(1, 2, 0), q02 = k(0, 0, 2) + rs * k(1, 0, 2);
+    const float q11 = k(0, 1, 1) + rs * k(1, 1, 1), q21 = r * k(0, 2, 1), q12 = r * k(0, 1, 2);
+    constexpr float w = 1.f / 6.f;
+    const float s00 = w * (q00 + t * (q20 + q02)), s10 = w * t * (q10 + t * q12), s01 = w * t * (q01 + t * q21);
+    acc[A_RHO] += s00;
+    acc[A_JX + AX] += s * s00;
+    acc[A_JX + P] += s10;
+    acc[A_JX + Q] += s01;
+    acc[aslot(AX, AX)] += s00;
+    acc[aslot(P, P)] += w * t * (q00 + q20 + t * q02);
+    acc[aslot(Q, Q)] += w * t * (q00 + q02 + t * q20);
+    acc[aslot(AX, P)] += s * s10;
+    acc[aslot(AX, Q)] += s * s01;
+    acc[aslot(P, Q)] += (w / 9.f) * q11;
 }
 
-// colour of one (cy, cz) group, as an increment over the target's own
-// phi: w ((phi_s - phi_t)(1 + P') + (B.c)/|c|) summed over cx.  Uniform
-// colour regions then keep phi exactly.
-template <int CYv, int CZv>
-__device__ __forceinline__ void col_group(float* acc, float ha, float hc, float hb, float Ex, float Ey, float Ez,
-                                          float By0, float Bz0) {
-    constexpr int cE = 1 + CYv * CYv + CZv * CZv, cC = CYv * CYv + CZv * CZv;
-    constexpr float wE = w1d(1) * w1d(CYv) * w1d(CZv), wC = w1d(0) * w1d(CYv) * w1d(CZv);
-    float r = Ex;
-    if (CYv) r += CYv > 0 ? Ey : -Ey;
-    if (CZv) r += CZv > 0 ? Ez : -Ez;
-    // summed in units of wE (wC = 4 wE), one weighting into the accumulator
-    float v = fmaf(wC / wE, hc, ha + hb);
-    v = fmaf(invlen(cE), r, v);
-    if (cC) {
-        float rc = 0.f;
-        if (CYv) rc += CYv > 0 ? By0 : -By0;
-        if (CZv) rc += CZv > 0 ? Bz0 : -Bz0;
-        v = fmaf((wC / wE) * invlen(cC), rc, v);
-    }
-    acc[A_COL] = fmaf(wE, v, acc[A_COL]);
+// The same of the three populations with c = s along axis AX and c = t along
+// axis BX, taken away (they belong to two faces).
+template <int AX, int BX, class Acc>
+__device__ __forceinline__ void edge_sub(const float* K, float s, float t, float r, const Acc& acc) {
+    constexpr int CX = 3 - AX - BX;
+    constexpr float w = -1.f / 36.f, th = 1.f / 3.f;
+    auto k = [&](int i, int j, int n) {
+        return K[kslot(AX == 0 ? i : BX == 0 ? j : n, AX == 1 ? i : BX == 1 ? j : n, AX == 2 ? i : BX == 2 ? j : n)];
+    };
+    const float rs = r * s, rt = r * t;
+    const float q0 = k(0, 0, 0) + k(2, 0, 0) + k(0, 2, 0) + rs * (k(1, 0, 0) + k(1, 2, 0)) + rt * (k(0, 1, 0) + k(2, 1, 0)) + rs * rt * k(1, 1, 0);
+    const float q1 = r * (k(0, 0, 1) + k(2, 0, 1) + k(0, 2, 1) + rs * k(1, 0, 1) + rt * k(0, 1, 1) + rs * rt * k(1, 1, 1));
+    const float q2 = k(0, 0, 2) + rs * k(1, 0, 2) + rt * k(0, 1, 2);
+    const float e0 = w * (q0 + th * q2), e1 = w * th * q1;
+    acc[A_RHO] += e0;
+    acc[A_JX + AX] += s * e0;
+    acc[A_JX + BX] += t * e0;
+    acc[A_JX + CX] += e1;
+    acc[aslot(AX, AX)] += e0;
+    acc[aslot(BX, BX)] += e0;
+    acc[aslot(CX, CX)] += w * th * (q0 + q2);
+    acc[aslot(AX, BX)] += s * t * e0;
+    acc[aslot(AX, CX)] += s * e1;
+    acc[aslot(BX, CX)] += t * e1;
 }
 
-// All populations that leave the source row y - CYv of plane s and land on
-// the column's targets in planes s-1 (accm), s (acc0), s+1 (accp).  Kc
-// points at the column's own node in the coefficient tile; phm, ph0, php
-// are the column's own phi in the three target planes (colour mode).
-template <int MODE, int CYv>
-__device__ __forceinline__ void pull_row(const CNode& Kc, float* accm, float* acc0, float* accp,
-                                         float phm, float ph0, float php) {
-    const Src<1, CYv> sa{Kc.at(-(CYv * CW + 1))};   // source of cx = +1 (x - 1)
-    const Src<0, CYv> sz{Kc.at(-(CYv * CW))};       // source of cx = 0
-    const Src<-1, CYv> sb{Kc.at(-(CYv * CW - 1))};  // source of cx = -1 (x + 1)
-    float am, a0, ap, cm, c0, cp, bm, b0, bp;
-    {
-        float2 pm, p0, pp;
-        SrcPair<CYv>{sa, sb}.eval(pm, p0, pp);
-        am = pm.x; bm = pm.y; a0 = p0.x; b0 = p0.y; ap = pp.x; bp = pp.y;
-    }
-    sz.eval(cm, c0, cp);
-    acc_group<CYv, -1>(accm, am, cm, bm);
-    acc_group<CYv, 0>(acc0, a0, c0, b0);
-    acc_group<CYv, 1>(accp, ap, cp, bp);
+// Half-way bounce-back f_c(x) = f^post_{-c}(x) at a node with several
+// bounce-back faces (bits mask): the faces' populations, less those of their
+// edges, counted twice, and with three faces the corner's again.
+template <int MODE, class Acc>
+__device__ __forceinline__ void bounce_target(const float* K, unsigned mask, const Acc& acc) {
+    const float sx = mask & 1u ? 1.f : -1.f, sy = mask & 4u ? 1.f : -1.f, sz = mask & 16u ? 1.f : -1.f;
+    const bool fx = mask & 3u, fy = mask & 12u, fz = mask & 48u;
+    const float bx = sx * K[K_C1], by = sy * K[K_C2], bz = sz * K[K_C3];
+    if (fx) face_sum<0>(K, sx, -1.f, acc);
+    if (fy) face_sum<1>(K, sy, -1.f, acc);
+    if (fz) face_sum<2>(K, sz, -1.f, acc);
+    if (fx && fy) edge_sub<0, 1>(K, sx, sy, -1.f, acc);
+    if (fx && fz) edge_sub<0, 2>(K, sx, sz, -1.f, acc);
+    if (fy && fz) edge_sub<1, 2>(K, sy, sz, -1.f, acc);
+    if (fx && fy && fz)
+        acc_dir_rt(acc, (int)sx, (int)sy, (int)sz, (1.f / 216.f) * eval_P(K, 1, -(int)sx, -(int)sy, -(int)sz));
     if (MODE == TSLB_MODE_COLOUR) {
-        const float pa = sa.L(K_C0), pz = sz.L(K_C0), pb = sb.L(K_C0);
-        // recolouring sums over the cx = +1 / -1 sources
-        const float Ex = sa.L(K_C1) - sb.L(K_C1);
-        const float Ey = CYv ? sa.L(K_C2) + sb.L(K_C2) : 0.f;
-        const float Ez = sa.L(K_C3) + sb.L(K_C3);
-        const float By0 = CYv ? sz.L(K_C2) : 0.f;
-        const float Bz0 = sz.L(K_C3);
-        // (phi_s - phi_t)(1 + P') for the three sources and the three target planes
-        auto h = [](float ps, float pt, float P) { const float d = ps - pt; return fmaf(d, P, d); };
-        col_group<CYv, -1>(accm, h(pa, phm, am), h(pz, phm, cm), h(pb, phm, bm), Ex, Ey, Ez, By0, Bz0);
-        col_group<CYv, 0>(acc0, h(pa, ph0, a0), h(pz, ph0, c0), h(pb, ph0, b0), Ex, Ey, Ez, By0, Bz0);
-        col_group<CYv, 1>(accp, h(pa, php, ap), h(pz, php, cp), h(pb, php, bp), Ex, Ey, Ez, By0, Bz0);
-        if (CYv == 0) {
-            // rest population: f_0 += delta0 (perturbation with B_0 = -10/27); its
-            // colour is the target's own, so it adds no colour increment
-            acc0[A_RHO] += sz.L(K_C4);
-        }
+        // the reflected populations carry the target's own colour: only the recolouring terms
+        constexpr float r2 = 0.70710678118654752f, r3 = 0.57735026918962576f;
+        constexpr float wf = (16.f + 16.f * r2 + 4.f * r3) / 216.f, we = (4.f * r2 + 2.f * r3) / 216.f;
+        float v = (fx ? wf * bx : 0.f) + (fy ? wf * by : 0.f) + (fz ? wf * bz : 0.f);
+        if (fx && fy) v -= we * (bx + by);
+        if (fx && fz) v -= we * (bx + bz);
+        if (fy && fz) v -= we * (by + bz);
+        if (fx && fy && fz) v += (r3 / 216.f) * (bx + by + bz);
+        // sources behind an x or y face were visited as nodes of phi 0
+        const float u = (fx && fy ? 11.f / 36.f : fx || fy ? 1.f / 6.f : 0.f) * (fz ? 5.f / 6.f : 1.f);
+        acc[A_COL] += u * K[K_C0] - v;
+    }
+    // phase field: the axis directions
+    if (MODE == TSLB_MODE_PHASEFIELD) {
+        if (fx) acc[A_COL] += K[K_C0] - bx;
+        if (fy) acc[A_COL] += K[K_C0] - by;
+        if (fz) acc[A_COL] += K[K_C0] - bz;
+    }
+}
+
+// Populations entering a node from behind one velocity or pressure face f: all
+// nine at once.  K: the node's coefficients, m its
+// moments.
+template <int MODE, class Acc>
+__device__ __forceinline__ void face_target(const StepArgs& a, const float* K, const float* m, float dt, int f, const Acc& acc) {
+    const FaceBC& fb = a.face[f];
+    const int ax = f >> 1;
+    const float s = f & 1 ? -1.f : 1.f, pht = K[K_C0];
+    // colour mode: a source behind an x or y face was visited as a node of phi 0
+    if (MODE == TSLB_MODE_COLOUR && ax < 2) acc[A_COL] += (1.f / 6.f) * pht;
+    // f^eq(rho, Ub) + (1 - omega) w a^neq(Pi, u): density 1 and the node's velocity
+    // and phi at a pressure outlet
+    const bool pressure = fb.kind == TSLB_BC_PRESSURE;
+    const float phib = pressure || fb.phi < -2.f ? m[F_PHI] : fb.phi;
+    float omega = a.omega_pf;
+    if (MODE == TSLB_MODE_COLOUR) {
+        const float ca = 0.5f * (1.f + m[F_PHI]), cb = 0.5f * (1.f - m[F_PHI]);
+        const float nu = 1.f / (ca * a.inv_nu_a + cb * a.inv_nu_b);
+        omega = 2.f / (6.f * nu + 1.f + 2.f * dt);
+    }
+    const float U = pressure ? m[F_U] : fb.u[0], V = pressure ? m[F_V] : fb.u[1], W = pressure ? m[F_W] : fb.u[2];
+    float Kb[K_XYZ + 1];
+    coefs_moments(pressure ? 0.f : m[F_D], m, U, V, W, 1.f - omega, Kb);
+    const float r0 = acc[A_RHO];
+    if (ax == 0) face_sum<0>(Kb, s, 1.f, acc);
+    else if (ax == 1) face_sum<1>(Kb, s, 1.f, acc);
+    else face_sum<2>(Kb, s, 1.f, acc);
+    if (MODE == TSLB_MODE_COLOUR) {
+        const float dphi = phib - pht;
+        acc[A_COL] += dphi * (1.f / 6.f + (acc[A_RHO] - r0));
     } else if (MODE == TSLB_MODE_PHASEFIELD) {
-        // phase field g (D3Q7): axis directions and the rest population
-        if (CYv == 0) {
-            const float g0 = sz.L(K_C0), gz = sz.L(K_C3);
-            accm[A_COL] += g0 - gz;                        // q = 6, (0,0,-1)
-            accp[A_COL] += g0 + gz;                        // q = 5, (0,0,+1)
-            acc0[A_COL] += sa.L(K_C0) + sa.L(K_C1);        // q = 1 from x - 1
-            acc0[A_COL] += sb.L(K_C0) - sb.L(K_C1);        // q = 2 from x + 1
-            acc0[A_COL] = fmaf(2.f, g0, acc0[A_COL]);      // q = 0: p0g phi = 2 G0
-        } else {
-            acc0[A_COL] += sz.L(K_C0) + CYv * sz.L(K_C2);  // q = 3 / 4
-        }
+        // g entering from the face (:984-986, :1044-1045)
+        acc[A_COL] += 0.125f * phib * (1.f + 3.f * s * fb.u[ax]);
     }
 }
 
 // Regularized or bounce-back populations entering target (x,y,z) from
-// behind non-periodic faces; Kp holds the target's own coefficients.
-template <int MODE, class T, bool TAU = false, bool SOLID = false>
-__device__ void boundary_target_k(const StepArgs& a, const float* Kp, unsigned mask, int x, int y, int z, float* acc) {
+// behind non-periodic faces or from interior solids, direction by direction,
+// added to acc (in shared memory: registers are short where this runs); Kp holds
+// the target's own coefficients.  The general path, for edges of faces of
+// different kinds, inlets, outlets and interior solids; single walls and
+// bounce-back edges have closed sums above (a 173 x 59 x 91 Couette cell with
+// this path at its walls 70 us a step, with closed sums 52).
+template <int S>
+struct Strided {
+    float* p;
+    __device__ __forceinline__ float& operator[](int i) const { return p[i * S]; }
+};
+template <int MODE, class T, bool TAU, bool SOLID, class Acc>
+__device__ __forceinline__ void boundary_target(const StepArgs& a, const float* Kp, unsigned mask, int x, int y, int z,
+                                                const Acc& acc) {
     // colour mode accumulates colour increments over the target's own phi
     const float pht = Kp[K_C0];
     // own raw moments (velocity faces only)
@@ -371,58 +351,49 @@ __device__ void boundary_target_k(const StepArgs& a, const float* Kp, unsigned m
     }
 }
 
-// the same, with the target's coefficients read from the coefficient tile at Kc
-template <int MODE, class T, bool TAU = false, bool SOLID = false>
-__device__ __forceinline__ void boundary_target(const StepArgs& a, const CNode& Kc, unsigned mask, int x, int y,
-                                                int z, float* acc) {
-    float Kp[NCOEF];
-#pragma unroll
-    for (int c = 0; c < NCOEF; ++c) Kp[c] = coef_at(Kc, c);
-    boundary_target_k<MODE, T, TAU, SOLID>(a, Kp, mask, x, y, z, acc);
-}
+// ---- tile geometry ----
+constexpr int LXV = 30;       // target columns of a warp: lanes 1 .. 30 (lanes 0 and 31 are sources only)
+// Warps of a block, W: 16 (one block on an SM) or 8 (two, for lattices whose
+// rows or planes do not fill 16).
+constexpr int BIGW = 16, SMALLW = 8;
+constexpr int NMOM = NF - 1;  // moments read per node (phi comes from the phi ring)
 
-// ---- shared-memory staging geometry ----
-// Moments and phi are staged with the tile's x range widened to whole
-// 16-byte chunks of EPC elements: columns x0-EPC .. x0+TX+EPC-1.
-constexpr int NTHR = TX * TY;
-constexpr int NHALO = CAREA - NTHR;           // coefficient nodes on the tile rim (84)
-constexpr int NMOM = NF - 1;                  // moments staged per node (phi comes from the phi ring)
-// Phi rows staged beyond the tile in y (and planes held beyond the source
-// plane in z): colour mode reads the gradient at the coefficient nodes (the
-// tile plus a one-node rim), 2; the phase field also the normals of their
-// neighbours for the curvature, 3.
-__host__ __device__ constexpr int phi_halo(int mode) { return mode == TSLB_MODE_PHASEFIELD ? 3 : 2; }
-template <int ES, int PHR = 2>   // element size in bytes, phi halo
-struct Geo {
-    static constexpr int EPC = 16 / ES;               // elements per 16-byte chunk
-    static constexpr int SW = TX + 2 * EPC;           // staged row width
-    static constexpr int OFF = EPC - 1;               // staged column of tile column 0 (x0 - 1)
-    static constexpr int NCH = SW / EPC;              // chunks per row
-    static constexpr int MROWS = CH;                  // moment rows: y0-1 .. y0+TY
-    static constexpr int PROWS = TY + 2 * PHR;        // phi rows: y0-PHR .. y0+TY+PHR-1
-    static constexpr int MAREA = MROWS * SW, PAREA = PROWS * SW;
-    static constexpr int MCELLS = MROWS * NCH;        // 16-byte cells of one staged moment plane
-    static constexpr int MGROUPS = NTHR / MCELLS;     // thread (g, cell) copies fields g, g + MGROUPS, ...
-    static constexpr int MFIELDS = (NMOM + MGROUPS - 1) / MGROUPS;
-    static_assert(MGROUPS >= 1, "a staged moment plane has more cells than the block has threads");
-    static constexpr int PCOPIES = PROWS * NCH;
-    static constexpr int PELEMS = PROWS * SW;
-    static constexpr int PEROUNDS = (PELEMS + NTHR - 1) / NTHR;
+// Phi rows and columns held beyond the block's source nodes: colour mode
+// reads the gradient at the source nodes, 1; the phase field also the normals
+// of their neighbours for the curvature, 2.  The phi planes held ahead of the
+// source plane are one more.
+__host__ __device__ constexpr int phi_rim(int mode) { return mode == TSLB_MODE_PHASEFIELD ? 2 : 1; }
+// Ring slots: plane z sits in slot z & (RING - 1).  While the slowest warp
+// still reads planes s-1 .. s+1 (colour; the phase field from s-2 on) the
+// fastest may already write plane s+3 (phase field s+4).
+constexpr int RING = 8;
+// A row of 32 source nodes is read as the 16-byte chunks that cover it: ROWE
+// elements from its start rounded down to a chunk.
+constexpr int ROWE = 40, MROW = ROWE * 4;   // elements, and bytes kept for a row of moments
+// Shared memory of a block: y values exchanged between warps, quads
+// [parity][direction][k][row][lane]; moments read ahead, [parity][field][row]
+// of MROW bytes, and the tau correction, [parity][thread]; the phi ring's rim
+// nodes, [2][thread] (place, offset); the moments of populations from behind
+// faces, [NACC][thread]; sources of the chunk reads, [2][thread]; the phi ring;
+// phase field: the curvature work list (the candidate nodes' tile indices for
+// two planes, their curvatures, two counts).  What is used once a plane is
+// kept here rather than in registers.
+template <int MODE, int W>
+struct Smem {
+    static constexpr int NT = 32 * W;
+    static constexpr int RAREA = ROWE * (W + 2 * phi_rim(MODE));
+    static constexpr int exch = 0;
+    static constexpr int mom = exch + 2 * 2 * 3 * NT * 16;
+    static constexpr int dt = mom + 2 * NMOM * W * MROW;
+    static constexpr int rim = dt + 2 * NT * 4;
+    static constexpr int bnd = rim + (MODE != TSLB_MODE_SINGLE ? 2 * NT * 8 : 0);
+    static constexpr int src = bnd + NACC * NT * 4;
+    static constexpr int ring = src + 2 * NT * 8;
+    static constexpr int curv = ring + (MODE != TSLB_MODE_SINGLE ? RING * RAREA * 4 : 0);
+    static constexpr int list = curv + (MODE == TSLB_MODE_PHASEFIELD ? NT * 4 : 0);
+    static constexpr int count = list + (MODE == TSLB_MODE_PHASEFIELD ? 2 * NT * 2 : 0);
+    static constexpr int bytes = count + (MODE == TSLB_MODE_PHASEFIELD ? 16 : 0);
 };
-
-// Phi ring: slot z & (PRING - 1) holds phi plane z.  Iteration s stages plane
-// s+PHR while other threads may still read planes from s-PHR on (the previous
-// iteration's pull or curvature), so the ring holds at least 2 PHR + 1 planes.
-constexpr int PRING = 8;
-// Phase field: the curvature work list of the block (section 4 of step_block):
-// the candidate nodes' tile indices for two planes, their curvatures, two counts
-constexpr size_t CURV_LIST_BYTES = sizeof(float) * CAREA + sizeof(unsigned short) * 2 * CAREA + sizeof(int) * 2;
-__host__ __device__ constexpr size_t step_smem_bytes_es(int mode, int es) {
-    return sizeof(float) * 2 * NCOEF * CAREA + (size_t)es * 2 * NMOM * CH * (TX + 2 * (16 / es)) +
-           (mode != TSLB_MODE_SINGLE ? (size_t)es * PRING * (TY + 2 * phi_halo(mode)) * (TX + 2 * (16 / es)) : 0) +
-           (mode == TSLB_MODE_PHASEFIELD ? CURV_LIST_BYTES : 0);
-}
-__host__ __device__ constexpr size_t step_smem_bytes(int mode) { return step_smem_bytes_es(mode, 4); }
 
 // gradient 3 sum_i p_i c_i phi(x+c_i) of one node (Ar1) or two (Ar2) from
 // phi planes held in shared memory: P(dz, dx, dy) returns phi at offset
@@ -452,12 +423,11 @@ __device__ __forceinline__ void grad_v(LD P, typename Ar::V g[3]) {
     g[2] = Ar::fma(c3, z3, Ar::fma(c2, z2, Ar::mul(c1, z1)));
 }
 // one node; pm, p0, pp point at it in planes z-1, z, z+1 (row pitch SWv).
-// fp16 storage: the caller multiplies the result by the phi scale.
-template <int SWv, class T>
-__device__ __forceinline__ void grad_smem(const T* pm, const T* p0, const T* pp, float g[3]) {
+template <int SWv>
+__device__ __forceinline__ void grad_smem(const float* pm, const float* p0, const float* pp, float g[3]) {
     grad_v<Ar1>([&](int dz, int dx, int dy) {
-        const T* pl = dz < 0 ? pm : dz > 0 ? pp : p0;
-        return Stor<T>::ld(pl[dy * SWv + dx]);
+        const float* pl = dz < 0 ? pm : dz > 0 ? pp : p0;
+        return pl[dy * SWv + dx];
     }, g);
 }
 
@@ -478,19 +448,14 @@ __device__ __forceinline__ typename Ar::V pf_indicator(typename Ar::V phi, const
     return Ar::mul(Ar::mul(phi, Ar::sub(Ar::c(1.f), phi)), nn);
 }
 
-template <int SWv, class T>
-__device__ __forceinline__ void pf_normal(const T* ring, int parea, int z, int pi, const StepArgs& a, float n[3]) {
-    const T* p0 = ring + (z & (PRING - 1)) * parea + pi;
-    const T* pm = ring + ((z - 1) & (PRING - 1)) * parea + pi;
-    const T* pp = ring + ((z + 1) & (PRING - 1)) * parea + pi;
+template <int SWv>
+__device__ __forceinline__ void pf_normal(const float* ring, int parea, int z, int pi, float n[3]) {
+    const float* p0 = ring + (z & (RING - 1)) * parea + pi;
+    const float* pm = ring + ((z - 1) & (RING - 1)) * parea + pi;
+    const float* pp = ring + ((z + 1) & (RING - 1)) * parea + pi;
     grad_smem<SWv>(pm, p0, pp, n);
-    if constexpr (std::is_same<T, __half>::value) {
-        n[0] = __fmul_rn(n[0], a.iscale[F_PHI]); n[1] = __fmul_rn(n[1], a.iscale[F_PHI]);
-        n[2] = __fmul_rn(n[2], a.iscale[F_PHI]);
-    }
     normalize_v<Ar1>(n);
 }
-
 
 struct XYNode {
     int off;      // gx + nx * gy (wrapped/clamped)
@@ -516,9 +481,8 @@ __device__ __forceinline__ XYNode xy_node(const StepArgs& a, int gx, int gy, boo
 // butterfly sums the 26 terms; every lane returns the sum.  z is the source
 // plane (ring index), gz its lattice plane, pi the node's staged offset and
 // (gx, gy) its lattice coordinates (may lie beyond a periodic face).
-static_assert(TX == 32, "a warp is one tile row: the lane is threadIdx.x");
-template <int SWv, bool SOLID, class T>
-__device__ float node_curvature(const T* ring, int parea, int z, int pi, int gx, int gy, int gz, const StepArgs& a,
+template <int SWv, bool SOLID>
+__device__ float node_curvature(const float* ring, int parea, int z, int pi, int gx, int gy, int gz, const StepArgs& a,
                                 bool xper, bool yper, bool zper) {
     const int lane = threadIdx.x;
     const int j = lane < 13 ? lane : lane + 1;   // 3 x 3 x 3 index of the neighbour, the centre (13) skipped
@@ -530,206 +494,353 @@ __device__ float node_curvature(const T* ring, int parea, int z, int pi, int gx,
     float t = 0.f;
     if (ok) {
         float n[3];
-        pf_normal<SWv>(ring, parea, z + dz, pi + dy * SWv + dx, a, n);
-        t = wclass(dx * dx + dy * dy + dz * dz) * ((float)dx * n[0] + (float)dy * n[1] + (float)dz * n[2]);
+        pf_normal<SWv>(ring, parea, z + dz, pi + dy * SWv + dx, n);
+        t = __fmul_rn(wclass(dx * dx + dy * dy + dz * dz),
+                      __fmaf_rn((float)dz, n[2], __fmaf_rn((float)dy, n[1], __fmul_rn((float)dx, n[0]))));
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return -3.f * t;
+    for (int o = 16; o > 0; o >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+    return __fmul_rn(-3.f, t);
 }
 
-__device__ __forceinline__ void cp_async4(float* sdst, const float* gsrc) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gsrc) : "memory");
+using V2 = Ar2::V;
+
+// The value of the node at x - 1 (lo) and x + 1 (hi): the neighbouring lanes', or
+// with the whole periodic axis in a warp any two lanes'.
+struct ShflNext {
+    __device__ __forceinline__ float lo(float v) const { return __shfl_up_sync(0xffffffffu, v, 1); }
+    __device__ __forceinline__ float hi(float v) const { return __shfl_down_sync(0xffffffffu, v, 1); }
+};
+struct ShflWrap {
+    int lm, lp;
+    __device__ __forceinline__ float lo(float v) const { return __shfl_sync(0xffffffffu, v, lm); }
+    __device__ __forceinline__ float hi(float v) const { return __shfl_sync(0xffffffffu, v, lp); }
+};
+
+// x sums of one monomial cy^j cz^k of P': the polynomial q0 + q1 cx + q2 cx^2
+// (NI coefficients) of the nodes at x - cx, weighted 1, 4, 1 and by cx^a:
+// T, D, S for a = 0, 1, 2; C (colour) as T with the factor phi(x - cx) - phi(x).
+// Held in pairs, as the y and z sums treat all four alike.
+struct XSum {
+    V2 td, sc;
+};
+template <int NI, bool COL, bool ONE, class SH>
+__device__ __forceinline__ XSum xsum(float q0, float q1, float q2, float dm, float dp, const SH& sh) {
+    using A = Ar1;
+    float Pp = q0, Pm = q0;
+    if (NI == 2) { Pp = A::add(q0, q1); Pm = A::sub(q0, q1); }
+    if (NI == 3) { const float t = A::add(q0, q2); Pp = A::add(t, q1); Pm = A::sub(t, q1); }
+    const float a = sh.lo(Pp), b = sh.hi(Pm);
+    XSum r;
+    const float S = A::add(a, b);
+    r.td = make_float2(A::fma(4.f, q0, S), A::sub(a, b));
+    // ONE: the constant 1 of 1 + P' belongs to this monomial
+    const float C = !COL ? 0.f : ONE ? A::add(A::fma(dm, a, dm), A::fma(dp, b, dp)) : A::fma(dp, b, A::mul(dm, a));
+    r.sc = make_float2(S, C);
+    return r;
 }
-__device__ __forceinline__ void cp_async16s(unsigned sa, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
+
+// A pair of polynomials in cy, q0 + q1 cy + q2 cy^2, at cy = 1 and -1
+struct YVal {
+    V2 p, m;
+};
+template <int NJ>
+__device__ __forceinline__ YVal yval(V2 q0, V2 q1, V2 q2) {
+    using A = Ar2;
+    const V2 t = NJ == 3 ? A::add(q0, q2) : q0;
+    return YVal{A::add(t, q1), A::sub(t, q1)};
+}
+
+// Write the 11 moments of one target node; chk is their sum.
+template <int MODE, class T, bool SOLID>
+__device__ __forceinline__ void store_target(const StepArgs& a, unsigned int id, long long plane, unsigned int sr_step,
+                                             const float* o, float chk) {
+    // single-component mode does not step phi (held at 1 in both buffers)
+    constexpr int nout = MODE == TSLB_MODE_SINGLE ? F_PHI : NF;
+    if (SOLID && bit_at(a.solid, id)) {
+        // interior solid nodes keep their moments
+#pragma unroll
+        for (int f = 0; f < NF; ++f) static_cast<T*>(a.fo[f])[id] = static_cast<const T*>(a.fi[f])[id];
+        return;
+    }
+    bool bad;
+    if constexpr (sizeof(T) == 2) {
+        // 16-bit storage: two fields per conversion (store_pair16), stochastic
+        // rounding seeded by the node (its index in the whole lattice) and the step
+        const unsigned int hnode = sr_node((unsigned int)(id + a.zoff * plane), sr_step);
+        float vmax = 0.f;
+#pragma unroll
+        for (int f = 0; f < nout; f += 2) {
+            const int g = f + 1 < nout ? f + 1 : f;
+            vmax = fmaxf(vmax, store_pair16<T>(a, id, f, g, o[f], o[g], a.sr, sr_field(hnode, f)));
+        }
+        // non-finite, or beyond the storage's range (NaN fails the comparison)
+        bad = !(vmax <= Stor16Max<T>::value);
+    } else {
+#pragma unroll
+        for (int f = 0; f < nout; ++f) static_cast<T*>(a.fo[f])[id] = o[f];
+        bad = !isfinite(chk);
+    }
+    if (bad) atomicOr(a.flags, 1u);
+}
+
+__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(sdst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(sdst)), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // T: storage type of the moment state (float, __nv_bfloat16, __half).
-// VEC: nx is a multiple of the 16-byte chunk, so chunks never straddle the
-// x faces and planes are staged with 16-byte cp.async copies.
-// One block's work: tile (bx, by) of columns and z chunk bz of lattice a.
+// One block's work: target planes z0 .. z1 - 1 of tile (bx, by) of lattice a.
+// TAU: the lattice has a per-node correction of the relaxation time (a.dtau).
 // SOLID: the lattice has interior solid nodes (bit masks a.solid, a.near).
-// PAIR: the warps holding rim nodes compute their two coefficient nodes at
-// once (coef_pair); the results are the same numbers either way, so a form
-// whose registers are short (the phase field inside an ensemble) leaves it.
-template <int MODE, bool VEC, class T, bool TAU = false, bool SOLID = false, bool PAIR = true>
-__device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, int bz) {
-    constexpr int PHR = phi_halo(MODE);
-    constexpr bool PHI = MODE != TSLB_MODE_SINGLE;   // phi is staged (colour, phase field)
-    using G = Geo<sizeof(T), PHR>;
-    constexpr int SW = G::SW, EPC = G::EPC, MAREA = G::MAREA, PAREA = G::PAREA;
+template <int MODE, class T, int W, bool TAU = false, bool SOLID = false>
+__device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, int z0, int z1) {
+    using A = Ar2;
+    using F = Ar1;
+    constexpr bool ASYNC = sizeof(T) == 4;   // phi copied by cp.async (16-bit phi is converted on the way)
+    constexpr bool COL = MODE == TSLB_MODE_COLOUR, PF = MODE == TSLB_MODE_PHASEFIELD, PHI = MODE != TSLB_MODE_SINGLE;
+    using SM = Smem<MODE, W>;
+    constexpr int RIM = phi_rim(MODE), RW = ROWE, RAREA = SM::RAREA, NEX = PF ? 2 : 1, NT = 32 * W;
+    // the row is the same for the whole warp: the shuffle tells the compiler
+    const int lane = threadIdx.x, wy = __shfl_sync(0xffffffffu, threadIdx.y, 0), tid = wy * 32 + lane;
     extern __shared__ float4 smem4[];
-    float* coef_base = reinterpret_cast<float*>(smem4);               // [2][NQUAD quads + pair][CAREA]
-    T* mst = reinterpret_cast<T*>(coef_base + 2 * NCOEF * CAREA);     // [2][NMOM][MROWS][SW]
-    T* phis = mst + 2 * NMOM * MAREA;                                 // [PRING][PROWS][SW] (not single)
-    // phase field: curvature work list (curvatures of plane s, candidates of planes s and s+1, their counts)
-    float* cq_curv = reinterpret_cast<float*>(phis + PRING * PAREA);  // [CAREA]
-    unsigned short* cq_list = reinterpret_cast<unsigned short*>(cq_curv + CAREA);   // [2][CAREA]
-    int* cq_n = reinterpret_cast<int*>(cq_list + 2 * CAREA);          // [2]
-    const T* gin = reinterpret_cast<const T*>(a.in);
-    T* gout = reinterpret_cast<T*>(a.out);
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-    const int x0 = bx * TX, y0 = by * TY;
-    const int z0 = a.zt0 + bz * a.zchunk;
-    const int z1 = min(z0 + a.zchunk, a.zt1);
-    const int X = x0 + tx, Y = y0 + ty;
-    const bool active = X < a.nx && Y < a.ny;
+    char* sm = reinterpret_cast<char*>(smem4);
+    float4* exch = reinterpret_cast<float4*>(sm + SM::exch);
+    char* mst = sm + SM::mom;
+    float* dts = reinterpret_cast<float*>(sm + SM::dt);
+    int2* exts = reinterpret_cast<int2*>(sm + SM::rim);
+    float* bnd = reinterpret_cast<float*>(sm + SM::bnd);
+    float* ring = reinterpret_cast<float*>(sm + SM::ring);
+    float* cq_curv = reinterpret_cast<float*>(sm + SM::curv);
+    unsigned short* cq_list = reinterpret_cast<unsigned short*>(sm + SM::list);
+    int* cq_n = reinterpret_cast<int*>(sm + SM::count);
     const bool xper = a.face[0].kind == TSLB_BC_PERIODIC;
     const bool yper = a.face[2].kind == TSLB_BC_PERIODIC;
     const bool zper = a.face[4].kind == TSLB_BC_PERIODIC;
-    const long long plane = (long long)a.nx * a.ny;
+    const unsigned plane = a.plane;
     // the step that seeds the stochastic rounding of 16-bit stores (an ensemble
     // advances a device counter after each step: its graph replays fixed arguments)
     const unsigned int sr_step = a.sr_counter ? *a.sr_counter : a.sr_step;
 
-    // faces the column touches (z faces are added per plane)
-    unsigned colmask = 0;
-    if (active) {
-        if (!xper && X == 0) colmask |= 1u;
-        if (!xper && X == a.nx - 1) colmask |= 2u;
-        if (!yper && Y == 0) colmask |= 4u;
-        if (!yper && Y == a.ny - 1) colmask |= 8u;
-    }
-
-    // coefficient nodes of this thread: its own column (r = 0) and one rim node (r = 1)
-    const bool has_rim = tid < NHALO;
-    XYNode cn0 = xy_node(a, X, Y, xper, yper), cn1;
-    const int ci0 = (ty + 1) * CW + (tx + 1);
-    int ci1;
-    {
-        int h = has_rim ? tid : 0, cx, cy;
-        if (h < CW) { cx = h; cy = 0; }
-        else if (h < 2 * CW) { cx = h - CW; cy = CH - 1; }
-        else if (h < 2 * CW + TY) { cx = 0; cy = h - 2 * CW + 1; }
-        else { cx = CW - 1; cy = h - 2 * CW - TY + 1; }
-        cn1 = xy_node(a, x0 - 1 + cx, y0 - 1 + cy, xper, yper);
-        ci1 = cy * CW + cx;
-    }
-    // position of a coefficient node (cx, cy) in the staged planes: moments
-    // row cy, column cx + OFF; phi row cy + PHR - 1, same column
-    const int mi0 = (ci0 / CW) * SW + (ci0 % CW) + G::OFF, mi1 = (ci1 / CW) * SW + (ci1 % CW) + G::OFF;
-    const int pi0 = mi0 + (PHR - 1) * SW, pi1 = mi1 + (PHR - 1) * SW;
-    const int nnodes = has_rim ? 2 : 1;
-
-    auto zwrap = [&](int z, bool& out) {
-        out = false;
-        if (z < 0 || z >= a.nz) { if (zper) return wrapi(z, a.nz); out = true; }
+    // this thread's node: column X, row Y
+    const int y0 = by * a.th, X = a.xwrap ? lane : bx * LXV - 1 + lane, Y = y0 - 1 + wy;
+    const int yend = min(y0 + a.th, a.ny);
+    const bool wact = Y <= yend;                // the row holds targets or sources of the tile
+    const bool wtgt = Y >= y0 && Y < yend;      // targets (the rim rows only send)
+    const bool valid = (a.xwrap ? lane < a.nx : (lane >= 1 && lane <= LXV && X < a.nx)) && wtgt;
+    const XYNode n0 = xy_node(a, X, Y, xper, yper);
+    // rows below and above, for the colour differences
+    const XYNode nd = xy_node(a, X, Y - 1, xper, yper), nu = xy_node(a, X, Y + 1, xper, yper);
+    // flags of the node: bits 0..3 the faces it touches (z faces are added per
+    // plane), then: it, its lower, its upper neighbour lies behind an x or y
+    // face; any node of the warp does
+    constexpr unsigned OUT0 = 64u, OUTD = 128u, OUTU = 256u, ANYOUT = 512u;
+    unsigned fl = (n0.out ? OUT0 : 0u) | (nd.out ? OUTD : 0u) | (nu.out ? OUTU : 0u);
+    if (!xper) fl |= (X == 0 ? 1u : 0u) | (X == a.nx - 1 ? 2u : 0u);
+    if (!yper) fl |= (Y == 0 ? 4u : 0u) | (Y == a.ny - 1 ? 8u : 0u);
+    if (__any_sync(0xffffffffu, n0.out)) fl |= ANYOUT;
+    // a plane's place in the lattice: wrapped, or the nearest plane behind a face
+    auto zclamp = [&](int z) {
+        if ((unsigned)z < (unsigned)a.nz) return z;
+        if (!zper) return z < 0 ? 0 : a.nz - 1;
+        while (z < 0) z += a.nz;
+        while (z >= a.nz) z -= a.nz;
         return z;
     };
+    auto zbehind = [&](int z) { return !zper && (unsigned)z >= (unsigned)a.nz; };
+    auto solid_bit = [&](unsigned out, int off, int gz) {
+        return (fl & out) || (SOLID && bit_at(a.solid, (unsigned)gz * plane + off));
+    };
 
-    // ---- staging of phi planes (colour and phase-field modes) ----
-    // VEC: copy j < PCOPIES is the 16-byte chunk (row j / NCH, chunk j % NCH);
-    // a chunk is either fully inside the domain (after the periodic wrap) or
-    // fully behind a non-periodic face, whose ghost values are computed.
-    int pch_off = 0, pch_dst = 0;
-    bool pch_out = true;
-    if (VEC && tid < G::PCOPIES) {
-        const int row = tid / G::NCH, ch = tid % G::NCH;
-        const XYNode nd = xy_node(a, x0 - EPC + EPC * ch, y0 - PHR + row, xper, yper);
-        pch_off = nd.off;
-        pch_out = nd.out;
-        pch_dst = row * SW + EPC * ch;
-    }
-    const T* pg0 = gin + F_PHI * a.N + pch_off;
-    const unsigned ps0 = (unsigned)__cvta_generic_to_shared(phis) + (unsigned)(pch_dst * sizeof(T));
-    auto ghost = [&](float v) { return cvt_out<T>(v, a, F_PHI); };
-    auto stage_phi = [&](int z) {
-        bool zout;
-        const int gz = zwrap(z, zout);
-        T* slot = phis + (z & (PRING - 1)) * PAREA;
-        const T* ph = gin + F_PHI * a.N + (long long)gz * plane;
-        if (VEC) {
-            if (tid < G::PCOPIES) {
-                T* dst = slot + pch_dst;
-                if (!pch_out && !zout) {
-                    cp_async16s(ps0 + (unsigned)((z & (PRING - 1)) * (PAREA * (int)sizeof(T))), pg0 + (long long)gz * plane);
-                } else {
-                    const int row = tid / G::NCH, ch = tid % G::NCH;
+    // ---- rows read as 16-byte chunks: FP32 or 16-bit rows of whole chunks (nx a
+    // multiple of EPC), the tile's columns (with the phi rim) inside a row ----
+    constexpr int EPC = 16 / (int)sizeof(T), CPR = ROWE / EPC;   // elements of a chunk, chunks of a row
+    const int X0 = X - lane;
+    const int Xm = X0 & ~(EPC - 1), Xp = (X0 - RIM) & ~3;        // first columns read (moments, phi)
+    const bool chunks = !a.xwrap && a.nx % EPC == 0 && X0 - RIM >= 0 && max(Xm, Xp) + ROWE <= a.nx;
+    const bool pchunks = PHI && ASYNC && chunks;
+    // inner: no node of the tile or its rim lies behind a face; then the planes
+    // whose neighbours and reads ahead are planes of the lattice as they stand
+    // take the iteration without those cases
+    const bool inner = !SOLID && !a.xwrap && (xper || (X0 - RIM >= 0 && X0 + 32 + RIM <= a.nx)) &&
+                       (yper || (y0 - 1 - RIM >= 0 && y0 - 1 + W + RIM <= a.ny));
+
+    // ---- phi ring: this thread fills its own node and up to NEX rim nodes ----
+    const int rx = pchunks ? X0 - RIM - Xp : 0;   // ring column of the tile's first phi column
+    const int ri = (wy + RIM) * RW + rx + lane + RIM;
+    // a mirrored wall repeats the nearest node, to which the offsets are clamped;
+    // other ghost values are computed
+    bool slow = n0.out;
 #pragma unroll
-                    for (int e = 0; e < EPC; ++e) dst[e] = ghost(phi_at<T>(a, x0 - EPC + EPC * ch + e, y0 - PHR + row, z));
-                }
+    for (int k = 0; k < NEX; ++k) {
+        int2 ex = make_int2(-1, n0.off);
+        constexpr int PW = 32 + 2 * RIM, side = 2 * RIM * PW;   // rim rows below and above, then side columns
+        const int e = tid + k * NT;
+        if (PHI && e < side + 2 * W * RIM) {
+            int r, c;
+            if (e < side) { r = e / PW; c = e % PW; if (r >= RIM) r += W; }
+            else { r = RIM + (e - side) / (2 * RIM); c = (e - side) % (2 * RIM); if (c >= RIM) c += 32; }
+            const XYNode n = xy_node(a, X0 + c - RIM, y0 - 1 + r - RIM, xper, yper);
+            ex = make_int2(r * RW + rx + c, n.off);
+            slow |= n.out;
+        }
+        if (PHI) exts[k * NT + tid] = ex;
+    }
+    slow = PHI && !a.phi_mirror && __any_sync(0xffffffffu, slow);
+    const T* phin = static_cast<const T*>(a.fi[F_PHI]);
+    struct PhiRow { float own, ex[NEX]; };
+    auto phi_store = [&](int z, const PhiRow& p) {
+        float* slot = ring + (z & (RING - 1)) * RAREA;
+        slot[ri] = p.own;
+#pragma unroll
+        for (int k = 0; k < NEX; ++k) {
+            const int d = exts[k * NT + tid].x;
+            if (d >= 0) slot[d] = p.ex[k];
+        }
+    };
+    // node by node
+    auto phi_load = [&](int z, PhiRow& p) {
+        const unsigned zoff = (unsigned)zclamp(z) * plane;
+        if (slow || (!a.phi_mirror && zbehind(z))) {
+            p.own = phi_at<T>(a, X, Y, z);
+#pragma unroll
+            for (int k = 0; k < NEX; ++k) {
+                const int d = exts[k * NT + tid].x;
+                p.ex[k] = d < 0 ? 0.f : phi_at<T>(a, X0 + d % RW - rx - RIM, y0 - 1 + d / RW - RIM, z);
+            }
+            if (ASYNC) phi_store(z, p);
+        } else if (ASYNC) {
+            float* slot = ring + (z & (RING - 1)) * RAREA;
+            cp_async4(slot + ri, phin + (zoff + n0.off));
+#pragma unroll
+            for (int k = 0; k < NEX; ++k) {
+                const int2 e = exts[k * NT + tid];
+                if (e.x >= 0) cp_async4(slot + e.x, phin + (zoff + e.y));
             }
         } else {
+            p.own = cvt_in<T>(__ldg(phin + (zoff + n0.off)), a, F_PHI);
 #pragma unroll
-            for (int r = 0; r < G::PEROUNDS; ++r) {
-                const int j = tid + r * NTHR;
-                if (j < G::PELEMS) {
-                    const int row = j / SW, col = j % SW;
-                    const XYNode nd = xy_node(a, x0 - EPC + col, y0 - PHR + row, xper, yper);
-                    if (!nd.out && !zout) {
-                        if constexpr (sizeof(T) == 4) cp_async4(reinterpret_cast<float*>(slot + j), reinterpret_cast<const float*>(ph + nd.off));
-                        else slot[j] = ph[nd.off];
-                    } else {
-                        slot[j] = ghost(phi_at<T>(a, nd.gx, nd.gy, z));
+            for (int k = 0; k < NEX; ++k) p.ex[k] = cvt_in<T>(__ldg(phin + (zoff + exts[k * NT + tid].y)), a, F_PHI);
+        }
+    };
+    // A warp's chunk reads of a plane: lanes below 30 read chunk lane % CPR of
+    // field lane / CPR + FPI i, i < NCHK, of their row of moments (cps: the
+    // source in plane 0); lanes 10 .. 29 the phi row and, in the warps that have
+    // one, a rim row (cpp).
+    constexpr int FPI = 30 / CPR, NCHK = (NMOM + FPI - 1) / FPI, mlast = CPR * (NMOM - FPI * (NCHK - 1));
+    const T** srcs = reinterpret_cast<const T**>(sm + SM::src) + tid;   // kept in shared memory: moments, phi
+    srcs[0] = static_cast<const T*>(a.in) + (lane / CPR) * a.N + (n0.off - X + Xm + (lane % CPR) * EPC);
+    char* cpd = mst + (lane / CPR) * W * MROW + wy * MROW + (lane % CPR) * 16;
+    const T* cpp = nullptr;
+    int cpr = 0;
+    if (pchunks && lane >= 10 && lane < 30) {
+        int r = wy + RIM;
+        bool has = true;
+        if (lane >= 20) {   // rim rows: below in the first warps, above in the last
+            has = wy < RIM || wy >= W - RIM;
+            r = wy < RIM ? wy : wy + 2 * RIM;
+        }
+        if (has) {
+            const XYNode n = xy_node(a, 0, y0 - 1 + r - RIM, xper, yper);
+            cpp = phin + (n.off + Xp + (lane % 10) * 4);
+            cpr = r * RW + (lane % 10) * 4;
+        }
+    }
+    srcs[NT] = cpp;
+    // two-dimensional parts of the gradient of one phi plane at the node: the x
+    // and y derivatives smoothed across, phi (c) and the smoothed phi less 36 c.
+    // Differences of phi come first, sums after: near a uniform phi the
+    // differences are exact, and the gradient's error is that of phi itself.
+    struct Sten { float dx, dy, ss, c; };
+    auto stencil = [&](int z) {
+        const float* r = ring + (z & (RING - 1)) * RAREA + ri - RW;
+        float d[3], s[3], c[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            c[k] = r[k * RW];
+            const float l = F::sub(r[k * RW - 1], c[k]), h = F::sub(r[k * RW + 1], c[k]);
+            d[k] = F::sub(h, l);
+            s[k] = F::add(h, l);
+        }
+        const float lo = F::sub(c[0], c[1]), hi = F::sub(c[2], c[1]);
+        Sten q;
+        q.dx = F::fma(4.f, d[1], F::add(d[0], d[2]));
+        q.dy = F::fma(6.f, F::sub(hi, lo), F::sub(s[2], s[0]));
+        q.ss = F::fma(6.f, F::add(hi, lo), F::fma(4.f, s[1], F::add(s[0], s[2])));
+        q.c = c[1];
+        return q;
+    };
+
+    // ---- reads ahead: phi of plane zp, then (mom) the moments and tau correction
+    // of plane z, as two groups of copies ----
+    auto load_ahead = [&](auto fast, int z, int zp, bool mom, PhiRow& p) {
+        constexpr bool FAST = decltype(fast)::value;
+        if (PHI && FAST) {
+            const unsigned zoff = (unsigned)zp * plane;
+            if (pchunks) {
+                const T* cpp = srcs[NT];
+                if (cpp) cp_async16(ring + cpr + (zp & (RING - 1)) * RAREA, cpp + zoff);
+            } else if (ASYNC) {
+                float* slot = ring + (zp & (RING - 1)) * RAREA;
+                cp_async4(slot + ri, phin + (zoff + n0.off));
+#pragma unroll
+                for (int k = 0; k < NEX; ++k) {
+                    const int2 e = exts[k * NT + tid];
+                    if (e.x >= 0) cp_async4(slot + e.x, phin + (zoff + e.y));
+                }
+            } else {
+                p.own = cvt_in<T>(__ldg(phin + (zoff + n0.off)), a, F_PHI);
+#pragma unroll
+                for (int k = 0; k < NEX; ++k) p.ex[k] = cvt_in<T>(__ldg(phin + (zoff + exts[k * NT + tid].y)), a, F_PHI);
+            }
+        } else if (PHI) {
+            if (pchunks && !slow && (a.phi_mirror || !zbehind(zp))) {
+                const T* cpp = srcs[NT];
+                if (cpp) cp_async16(ring + cpr + (zp & (RING - 1)) * RAREA, cpp + (unsigned)zclamp(zp) * plane);
+            } else {
+                phi_load(zp, p);
+            }
+        }
+        cp_async_commit();
+        if (mom) {
+            const unsigned zoff = (unsigned)(FAST ? z : zclamp(z)) * plane;
+            const int par = (z & 1) * NMOM * W * MROW;
+            if (chunks) {
+                const T* src = srcs[0] + zoff;
+                if (lane < 30) {
+#pragma unroll
+                    for (int i = 0; i < NCHK; ++i) {
+                        if (i < NCHK - 1 || lane < mlast) cp_async16(cpd + par + i * FPI * W * MROW, src);
+                        src += FPI * a.N;
                     }
                 }
-            }
-        }
-    };
-
-    // ---- staging of the 10 non-phi moments of plane z ----
-    // VEC: thread tid < MGROUPS MCELLS owns cell tid % MCELLS (row, chunk) of the
-    // staged plane and copies it for the fields tid / MCELLS + k MGROUPS; the
-    // addresses are fixed per thread, only the plane changes.
-    int mcell_dst = 0, mcell_off = 0, mfg = 0;
-    bool mcell_ok = false;
-    if (VEC && tid < G::MGROUPS * G::MCELLS) {
-        const int cell = tid % G::MCELLS, row = cell / G::NCH, ch = cell % G::NCH;
-        mfg = tid / G::MCELLS;
-        const XYNode nd = xy_node(a, x0 - EPC + EPC * ch, y0 - 1 + row, xper, yper);
-        mcell_off = nd.off;
-        mcell_ok = !nd.out;
-        mcell_dst = mfg * MAREA + row * SW + EPC * ch;
-    }
-    // per-thread staging bases: global (field group, cell) and shared (cell)
-    const T* mg0 = gin + mfg * a.N + mcell_off;
-    const long long mfstride = (long long)G::MGROUPS * a.N;
-    const unsigned ms0 = (unsigned)__cvta_generic_to_shared(mst) + (unsigned)(mcell_dst * sizeof(T));
-
-    auto stage_mom = [&](int z) {
-        bool zout;
-        const int gz = zwrap(z, zout);
-        if (zout) return;
-        T* dst = mst + (z & 1) * (NMOM * MAREA);
-        const T* src = gin + (long long)gz * plane;
-        if (VEC) {
-            if (mcell_ok) {
-                const unsigned d = ms0 + (unsigned)((z & 1) * (NMOM * MAREA * (int)sizeof(T)));
-                const T* g = mg0 + (long long)gz * plane;
+            } else {
+                // node by node: the 4-byte word that holds it
+                const unsigned id = zoff + n0.off;
+                char* st = mst + par + wy * MROW + lane * 4;
 #pragma unroll
-                for (int k = 0; k < G::MFIELDS; ++k) {
-                    if (G::MGROUPS * G::MFIELDS == NMOM || mfg + k * G::MGROUPS < NMOM)
-                        cp_async16s(d + (unsigned)(k * G::MGROUPS * MAREA * (int)sizeof(T)), g + k * mfstride);
-                }
+                for (int f = 0; f < NMOM; ++f)
+                    cp_async4(st + f * W * MROW, static_cast<const unsigned*>(a.fi[f]) + (sizeof(T) == 4 ? id : id >> 1));
             }
-        } else {
-            for (int r = 0; r < nnodes; ++r) {
-                const XYNode nd = r ? cn1 : cn0;
-                if (nd.out) continue;
-                const T* p = src + nd.off;
-                T* d = dst + (r ? mi1 : mi0);
-#pragma unroll
-                for (int f = 0; f < NMOM; ++f) {
-                    if constexpr (sizeof(T) == 4) cp_async4(reinterpret_cast<float*>(d + f * MAREA), reinterpret_cast<const float*>(p + f * a.N));
-                    else d[f * MAREA] = p[f * a.N];
-                }
-            }
+            if (TAU) cp_async4(dts + (z & 1) * NT + tid, a.dtau + (zoff + n0.off));
         }
+        cp_async_commit();
     };
-
-    // phi of the planes the first source plane z0 - 1 reads: z0 - PHR .. z0 + PHR - 2
-    if (PHI)
-        for (int z = z0 - PHR; z <= z0 + PHR - 2; ++z) stage_phi(z);
-    stage_mom(z0 - 1);
-    cp_async_commit();
-    if (MODE == TSLB_MODE_PHASEFIELD && tid == 0) cq_n[0] = cq_n[1] = 0;
-    cp_async_wait<0>();
-    __syncthreads();
+    // the node's moments from a plane read ahead (after the warp's copies have landed)
+    float m[NF], dt = 0.f;
+    const char* mrd = mst + wy * MROW + (chunks ? (X - Xm) * (int)sizeof(T) : lane * 4);
+    auto mom_take = [&](int z) {
+        const char* e = mrd + (z & 1) * NMOM * W * MROW;
+        if (sizeof(T) == 2 && !chunks) e += (((unsigned)zclamp(z) * plane + n0.off) & 1) * 2;
+#pragma unroll
+        for (int f = 0; f < NMOM; ++f) m[f] = cvt_in<T>(*reinterpret_cast<const T*>(e + f * W * MROW), a, f);
+        if (TAU) dt = dts[(z & 1) * NT + tid];
+    };
 
     // Phase field: the curvature of a plane's interface nodes is shared by all
     // warps of the block.  The coefficient phase of plane s lists the nodes of
@@ -737,321 +848,385 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     // indicator's threshold, a superset of the nodes where phi (1 - phi) |n|^2
     // exceeds it); the next coefficient phase, after the plane barrier, first
     // computes their curvatures warp by warp, then (one more barrier) the
-    // coefficients.  A node's position in its plane's list: slot0 / slot1.
-    int slot0 = -1, slot1 = -1;
+    // coefficients.  cslot: the node's position in its plane's list.
+    int cslot = -1;
     auto list_candidates = [&](int z) {
-        bool zs;
-        const int gzc = zwrap(z, zs);
-        if (zs) { slot0 = slot1 = -1; return; }
-        auto cand = [&](const bool has, const XYNode& nd, const int ci, const int pi) {
-            if (!has || nd.out || (SOLID && bit_at(a.solid, (long long)gzc * plane + nd.off))) return -1;
-            const float ph = cvt_in<T>(phis[(z & (PRING - 1)) * PAREA + pi], a, F_PHI);
-            if (!(ph * (1.f - ph) > 0.2f * (1.f - 1e-5f))) return -1;
-            const int e = atomicAdd(&cq_n[z & 1], 1);
-            cq_list[(z & 1) * CAREA + e] = (unsigned short)ci;
-            return e;
-        };
-        slot0 = cand(true, cn0, ci0, pi0);
-        slot1 = cand(has_rim, cn1, ci1, pi1);
+        cslot = -1;
+        if (zbehind(z) || !wact || solid_bit(OUT0, n0.off, zclamp(z))) return;
+        const float ph = ring[(z & (RING - 1)) * RAREA + ri];
+        if (!(ph * (1.f - ph) > 0.2f * (1.f - 1e-5f))) return;
+        cslot = atomicAdd(&cq_n[z & 1], 1);
+        cq_list[(z & 1) * NT + cslot] = (unsigned short)tid;
     };
-    if (MODE == TSLB_MODE_PHASEFIELD) {
+
+    // prologue: the phi planes the first source plane reads, its moments
+    for (int z = z0 - 1 - RIM; z <= z0 - 1 + RIM; ++z) {
+        PhiRow p;
+        if (PHI || z == z0 - 1 + RIM) load_ahead(std::false_type{}, z0 - 1, z, wact && z == z0 - 1 + RIM, p);
+        if (PHI && !ASYNC) phi_store(z, p);
+    }
+    if (PF && tid == 0) cq_n[0] = cq_n[1] = 0;
+    cp_async_wait<0>();
+    __syncthreads();
+    // gradient so far at planes s (x, y: planes s-1 and s; z: their difference) and
+    // s+1 (plane s; z: its smoothed phi gs, phi itself being in the ring)
+    float gx = 0.f, gy = 0.f, gz_ = 0.f, gx1 = 0.f, gy1 = 0.f, gs = 0.f;
+    // own phi (0 at nodes that send nothing) of one plane of the ring;
+    // of a plane behind a z face: the nearest plane's, so that it has no phi difference
+    auto own_phi = [&](int z) {
+        const int zc = zclamp(z);
+        float p = ring[((zbehind(z) ? zc : z) & (RING - 1)) * RAREA + ri];
+        if (SOLID || (fl & ANYOUT)) {
+            if (solid_bit(OUT0, n0.off, zc)) p = 0.f;
+        }
+        return p;
+    };
+    if (PHI) {
+        const Sten a1 = stencil(z0 - 2), a2 = stencil(z0 - 1);
+        gx = F::fma(4.f, a2.dx, a1.dx); gy = F::fma(4.f, a2.dy, a1.dy);
+        gx1 = a2.dx; gy1 = a2.dy;
+        gz_ = F::fma(36.f, F::sub(a2.c, a1.c), F::sub(a2.ss, a1.ss)); gs = a2.ss;
+    }
+    if (PF) {
         list_candidates(z0 - 1);
         __syncthreads();
     }
 
-    float accm[NACC], acc0[NACC], accp[NACC];
-#pragma unroll
-    for (int i = 0; i < NACC; ++i) { accm[i] = 0.f; acc0[i] = 0.f; accp[i] = 0.f; }
+    // partial sums of the targets, in units of 1/216.  Moments (a, b, c) in
+    // pairs: A = (00, 10), B = (20, colour), M = (01, 11) and 02 of a, b.
+    // Target s: M0* (c = 0), M1* (c = 1: 00 10 01), M2 (c = 2: 00);
+    // target s+1: U* (the same for every c).
+    const V2 zero2 = make_float2(0.f, 0.f);
+    V2 M0A = zero2, M0B = zero2, M0M = zero2, M1A = zero2, UA = zero2, UB = zero2, UM = zero2;
+    float M02 = 0.f, M1b = 0.f, M2 = 0.f, U02 = 0.f;
 
-    int buf = 0;
-    for (int s = z0 - 1; s <= z1; ++s) {
-        float* coef = coef_base + buf * (NCOEF * CAREA);
+    // source plane s.  FAST: an inner tile and plane (see `inner`)
+    auto iterate = [&](auto fast, const int s) {
+        constexpr bool FAST = decltype(fast)::value;
         const bool more = s < z1;
-        // ---- 0. prefetch: phi of plane s+PHR, moments of plane s+1 ----
-        if (PHI && more) stage_phi(s + PHR);
-        cp_async_commit();
-        if (more) stage_mom(s + 1);
-        cp_async_commit();
-        // non-VEC: this thread's own moment copies of plane s; VEC: every copy of
-        // plane s was waited for before the previous plane's pre-pull barrier
-        if (!VEC) cp_async_wait<2>();
-        // ---- 1. coefficients of source plane s: own column and one rim node ----
-        bool zsolid;
-        const int gz = zwrap(s, zsolid);
-        const T* ms = mst + (s & 1) * (NMOM * MAREA);
-        // a solid source plane sends nothing: no coefficients, no pull
-        auto coef_node = [&](const XYNode& nd, const int ci, const int mi, const int pi) {
-            float K[NCOEF];
-            // solid nodes (behind a face, or interior solids) send nothing
-            if (nd.out || (SOLID && bit_at(a.solid, (long long)gz * plane + nd.off))) {
-#pragma unroll
-                for (int c = 0; c < NCOEF; ++c) K[c] = 0.f;
-            } else {
-                float m[NF];
-#pragma unroll
-                for (int f = 0; f < NMOM; ++f) m[f] = cvt_in<T>(ms[f * MAREA + mi], a, f);
-                float g[3] = {0.f, 0.f, 0.f};
-                if (MODE == TSLB_MODE_COLOUR) {
-                    const T* p0 = phis + (s & (PRING - 1)) * PAREA + pi;
-                    const T* pm = phis + ((s - 1) & (PRING - 1)) * PAREA + pi;
-                    const T* pp = phis + ((s + 1) & (PRING - 1)) * PAREA + pi;
-                    m[F_PHI] = cvt_in<T>(*p0, a, F_PHI);
-                    grad_smem<SW>(pm, p0, pp, g);
-                    if constexpr (std::is_same<T, __half>::value) {
-                        g[0] = __fmul_rn(g[0], a.iscale[F_PHI]); g[1] = __fmul_rn(g[1], a.iscale[F_PHI]);
-                        g[2] = __fmul_rn(g[2], a.iscale[F_PHI]);
-                    }
-                } else {
-                    m[F_PHI] = 1.f;
-                }
-                node_coefs<MODE, TAU>(a, m, g, 0.f, K, TAU ? (long long)gz * plane + nd.off : 0);
-            }
-            store_coefs<MODE>(coef, ci, K);
+        auto neighbours = [&]() {
+            if constexpr (FAST) return ShflNext{};
+            else return ShflWrap{a.xwrap ? (lane == 0 ? a.nx - 1 : lane - 1) : max(lane - 1, 0),
+                                 a.xwrap && lane == a.nx - 1 ? 0 : min(lane + 1, 31)};
         };
-        // The warps that hold rim nodes (rows 0-2 of the tile: threads tid < NHALO)
-        // have two coefficient nodes per plane and set the length of the phase
-        // before the plane barrier.  They evaluate both at once on the paired
-        // FP32 instructions: lane x the own node, lane y the rim node (a thread
-        // without one repeats its own node in y and stores x alone).  Every
-        // operation rounds as in coef_node, so a node gets the same coefficients
-        // as an own node of one tile and as a rim node of another.
-        auto coef_pair = [&]() {
-            const XYNode nb = has_rim ? cn1 : cn0;
-            const int miB = has_rim ? mi1 : mi0, piB = has_rim ? pi1 : pi0;
-            Ar2::V m[NF], g[3] = {Ar2::c(0.f), Ar2::c(0.f), Ar2::c(0.f)};
-#pragma unroll
-            for (int f = 0; f < NMOM; ++f)
-                m[f] = make_float2(cvt_in<T>(ms[f * MAREA + mi0], a, f), cvt_in<T>(ms[f * MAREA + miB], a, f));
-            if (MODE == TSLB_MODE_COLOUR) {
-                const T* r0 = phis + (s & (PRING - 1)) * PAREA;
-                const T* rm = phis + ((s - 1) & (PRING - 1)) * PAREA;
-                const T* rp = phis + ((s + 1) & (PRING - 1)) * PAREA;
-                m[F_PHI] = make_float2(cvt_in<T>(r0[pi0], a, F_PHI), cvt_in<T>(r0[piB], a, F_PHI));
-                grad_v<Ar2>([&](int dz, int dx, int dy) {
-                    const T* pl = dz < 0 ? rm : dz > 0 ? rp : r0;
-                    const int o = dy * SW + dx;
-                    return make_float2(Stor<T>::ld(pl[pi0 + o]), Stor<T>::ld(pl[piB + o]));
-                }, g);
-                if constexpr (std::is_same<T, __half>::value) {
-                    const Ar2::V sc = Ar2::c(a.iscale[F_PHI]);
-                    g[0] = Ar2::mul(g[0], sc); g[1] = Ar2::mul(g[1], sc); g[2] = Ar2::mul(g[2], sc);
-                }
-            } else {
-                m[F_PHI] = Ar2::c(1.f);
-            }
-            const long long pz = (long long)gz * plane;
-            const Ar2::V dt = TAU ? make_float2(__ldg(a.dtau + pz + cn0.off), __ldg(a.dtau + pz + nb.off)) : Ar2::c(0.f);
-            Ar2::V K2[NCOEF];
-            node_coefs_v<MODE, TAU, Ar2>(a, m, g, Ar2::c(0.f), dt, K2);
-            // solid nodes (behind a face, or interior solids) send nothing
-            const bool s0 = cn0.out || (SOLID && bit_at(a.solid, pz + cn0.off));
-            const bool s1 = nb.out || (SOLID && bit_at(a.solid, pz + nb.off));
-            float K[NCOEF];
-#pragma unroll
-            for (int c = 0; c < NCOEF; ++c) K[c] = s0 ? 0.f : K2[c].x;
-            store_coefs<MODE>(coef, ci0, K);
-            if (has_rim) {
-#pragma unroll
-                for (int c = 0; c < NCOEF; ++c) K[c] = s1 ? 0.f : K2[c].y;
-                store_coefs<MODE>(coef, ci1, K);
-            }
-        };
-        // Phase field: the interface normal n = grad phi / (|grad phi| + 1e-9) of
-        // the node (recursive_2c_TSLB3D.f90:555-571) and, where the indicator
-        // phi (1 - phi) |n|^2 exceeds 0.2, the curvature -div n over the 26
-        // neighbours' normals (:614-629), taken from the block's work list.
-        auto coef_node_pf = [&](const XYNode& nd, const int ci, const int mi, const int pi, const int slot) {
-            float K[NCOEF];
-            if (nd.out || (SOLID && bit_at(a.solid, (long long)gz * plane + nd.off))) {
-#pragma unroll
-                for (int c = 0; c < NCOEF; ++c) K[c] = 0.f;
-            } else {
-                float m[NF], g[3];
-#pragma unroll
-                for (int f = 0; f < NMOM; ++f) m[f] = cvt_in<T>(ms[f * MAREA + mi], a, f);
-                const float phi = cvt_in<T>(phis[(s & (PRING - 1)) * PAREA + pi], a, F_PHI);
-                m[F_PHI] = phi;
-                pf_normal<SW>(phis, PAREA, s, pi, a, g);
-                const bool need = pf_indicator<Ar1>(phi, g) > 0.2f;
-                // a node that needs the curvature was listed as a candidate (slot >= 0)
-                const float curv = need && slot >= 0 ? cq_curv[slot] : 0.f;
-                node_coefs<MODE, TAU>(a, m, g, curv, K, TAU ? (long long)gz * plane + nd.off : 0);
-            }
-            store_coefs<MODE>(coef, ci, K);
-        };
-        // the same two nodes at once for the phase field (coef_node_pf per lane)
-        auto coef_pair_pf = [&]() {
-            const XYNode nb = has_rim ? cn1 : cn0;
-            const int miB = has_rim ? mi1 : mi0, piB = has_rim ? pi1 : pi0, slotB = has_rim ? slot1 : slot0;
-            Ar2::V m[NF], g[3];
-#pragma unroll
-            for (int f = 0; f < NMOM; ++f)
-                m[f] = make_float2(cvt_in<T>(ms[f * MAREA + mi0], a, f), cvt_in<T>(ms[f * MAREA + miB], a, f));
-            const T* r0 = phis + (s & (PRING - 1)) * PAREA;
-            const T* rm = phis + ((s - 1) & (PRING - 1)) * PAREA;
-            const T* rp = phis + ((s + 1) & (PRING - 1)) * PAREA;
-            const Ar2::V phi = make_float2(cvt_in<T>(r0[pi0], a, F_PHI), cvt_in<T>(r0[piB], a, F_PHI));
-            m[F_PHI] = phi;
-            grad_v<Ar2>([&](int dz, int dx, int dy) {
-                const T* pl = dz < 0 ? rm : dz > 0 ? rp : r0;
-                const int o = dy * SW + dx;
-                return make_float2(Stor<T>::ld(pl[pi0 + o]), Stor<T>::ld(pl[piB + o]));
-            }, g);
-            if constexpr (std::is_same<T, __half>::value) {
-                const Ar2::V sc = Ar2::c(a.iscale[F_PHI]);
-                g[0] = Ar2::mul(g[0], sc); g[1] = Ar2::mul(g[1], sc); g[2] = Ar2::mul(g[2], sc);
-            }
-            normalize_v<Ar2>(g);
-            const Ar2::V ind = pf_indicator<Ar2>(phi, g);
-            // a node that needs the curvature was listed as a candidate (slot >= 0)
-            const Ar2::V curv = make_float2(ind.x > 0.2f && slot0 >= 0 ? cq_curv[slot0] : 0.f,
-                                            ind.y > 0.2f && slotB >= 0 ? cq_curv[slotB] : 0.f);
-            const long long pz = (long long)gz * plane;
-            const Ar2::V dt = TAU ? make_float2(__ldg(a.dtau + pz + cn0.off), __ldg(a.dtau + pz + nb.off)) : Ar2::c(0.f);
-            Ar2::V K2[NCOEF];
-            node_coefs_v<MODE, TAU, Ar2>(a, m, g, curv, dt, K2);
-            const bool s0 = cn0.out || (SOLID && bit_at(a.solid, pz + cn0.off));
-            const bool s1 = nb.out || (SOLID && bit_at(a.solid, pz + nb.off));
-            float K[NCOEF];
-#pragma unroll
-            for (int c = 0; c < NCOEF; ++c) K[c] = s0 ? 0.f : K2[c].x;
-            store_coefs<MODE>(coef, ci0, K);
-            if (has_rim) {
-#pragma unroll
-                for (int c = 0; c < NCOEF; ++c) K[c] = s1 ? 0.f : K2[c].y;
-                store_coefs<MODE>(coef, ci1, K);
-            }
-        };
-        if (MODE == TSLB_MODE_PHASEFIELD) {
-            // curvatures of this plane's candidates, warp w taking entries w, w + 8, ...
-            // (the count is the same for every thread: the list was completed before
-            // the previous plane's barrier)
+        const auto sh = neighbours();
+        const bool zsolid = !FAST && zbehind(s);   // a solid source plane sends nothing
+        const int gz = FAST ? s : zclamp(s);
+        auto phi_of = [&](int z) { return FAST ? ring[(z & (RING - 1)) * RAREA + ri] : own_phi(z); };
+        float4* ex = exch + (s & 1) * (2 * 3 * NT);
+        // ---- 0. moments of the next plane, phi of the plane after the ring's last ----
+        cp_async_wait<0>();
+        __syncwarp();   // the warp's copies of the moments of plane s have landed
+        if (wact) mom_take(s);
+        PhiRow ph;
+        if (more) load_ahead(fast, s + 1, s + 1 + RIM, wact, ph);
+        // ---- curvatures of this plane's candidates, warp w taking entries w, w + nw, ...
+        // (the count is the same for every thread: the list was completed before
+        // the previous plane's barrier)
+        if (PF) {
             const int cnt = cq_n[s & 1];
             if (cnt > 0) {
-                for (int e = ty; e < cnt; e += TY) {
-                    const int ci = cq_list[(s & 1) * CAREA + e];
-                    const int cx = ci % CW, cy = ci / CW;
-                    const float k = node_curvature<SW, SOLID>(phis, PAREA, s, cy * SW + cx + G::OFF + (PHR - 1) * SW,
-                                                              x0 - 1 + cx, y0 - 1 + cy, gz, a, xper, yper, zper);
-                    if (tx == 0) cq_curv[e] = k;
+                for (int e = wy; e < cnt; e += W) {
+                    const int ci = cq_list[(s & 1) * NT + e];
+                    const int cx = ci & 31, cy = ci >> 5;
+                    const float k = node_curvature<RW, SOLID>(ring, RAREA, s, (cy + RIM) * RW + rx + cx + RIM, X0 + cx,
+                                                              y0 - 1 + cy, gz, a, xper, yper, zper);
+                    if (lane == 0) cq_curv[e] = k;
                 }
                 __syncthreads();
                 // every thread has read cnt; the next entries of this parity come after the plane barrier
                 if (tid == 0) cq_n[s & 1] = 0;
             }
         }
-        if (!zsolid) {
-            if constexpr (MODE == TSLB_MODE_PHASEFIELD) {
-                if (PAIR && ty * TX < NHALO) {
-                    coef_pair_pf();
-                } else {
-                    coef_node_pf(cn0, ci0, mi0, pi0, slot0);
-                    if (!PAIR && has_rim) coef_node_pf(cn1, ci1, mi1, pi1, slot1);
-                }
-            } else if (PAIR && ty * TX < NHALO) {
-                coef_pair();
+        // kept across the barrier: the sums at cy = 0 per k, own phi of plane s+1
+        V2 ktd[3], ksc[3];
+        float pc = 0.f, rest = 0.f, gzf = 0.f;
+        bool near = false;   // the target has populations from behind a face or from interior solids
+        if (wact) {
+            // ---- 1. coefficients ----
+            float g[3], K[NCOEF];
+            if (PHI) {
+                const Sten q = stencil(s + 1);
+                constexpr float k72 = 1.f / 72.f;
+                g[0] = F::mul(F::add(gx, q.dx), k72);
+                g[1] = F::mul(F::add(gy, q.dy), k72);
+                const float dz = F::fma(36.f, F::sub(q.c, ring[(s & (RING - 1)) * RAREA + ri]), F::sub(q.ss, gs));
+                g[2] = F::mul(F::add(gz_, dz), k72);
+                gz_ = dz; gs = q.ss;
+                gx = F::fma(4.f, q.dx, gx1); gx1 = q.dx;
+                gy = F::fma(4.f, q.dy, gy1); gy1 = q.dy;
+            }
+            bool iface = false;
+            if (COL) {
+                m[F_PHI] = pc = phi_of(s);
+                iface = coefs_colour<TAU>(a, m, g, dt, K);
+            } else if (PF) {
+                m[F_PHI] = ring[(s & (RING - 1)) * RAREA + ri];
+                normalize_v<F>(g);
+                // a node that needs the curvature was listed as a candidate
+                const float curv = pf_indicator<F>(m[F_PHI], g) > 0.2f && cslot >= 0 ? cq_curv[cslot] : 0.f;
+                coefs_shifted<true>(a, m, g, curv, K);
             } else {
-                coef_node(cn0, ci0, mi0, pi0);
-                if (!PAIR && has_rim) coef_node(cn1, ci1, mi1, pi1);
+                coefs_shifted<false>(a, m, g, 0.f, K);
+            }
+            // solid nodes (behind a face, or interior solids) send nothing
+            if (!FAST && (SOLID || (fl & ANYOUT) || zsolid)) {
+                if (zsolid || solid_bit(OUT0, n0.off, gz)) {
+#pragma unroll
+                    for (int c = 0; c < NCOEF; ++c) K[c] = 0.f;
+                }
+            }
+            // ---- populations from behind non-periodic faces, target plane s ----
+            if (!FAST && s >= z0 && s < z1) {
+                const unsigned mask = (fl & 15u) | (zper ? 0u : (s == 0 ? 16u : 0u) | (s == a.nz - 1 ? 32u : 0u));
+                near = valid && (mask || (SOLID && bit_at(a.near, (unsigned)s * plane + n0.off)));
+                if (near) {
+                    const Strided<NT> acc{bnd + tid};
+#pragma unroll
+                    for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+                    bool bounce = (mask & mask >> 1 & 0x15u) == 0;   // (one face of each axis)
+#pragma unroll
+                    for (int f = 0; f < 6; ++f)
+                        if (mask >> f & 1u) bounce = bounce && a.face[f].kind == TSLB_BC_BOUNCEBACK;
+                    const int f = __ffs(mask) - 1, kind = f >= 0 ? a.face[f].kind : TSLB_BC_PERIODIC;
+                    if (SOLID && bit_at(a.near, (unsigned)s * plane + n0.off)) {
+                        boundary_target<MODE, T, TAU, SOLID>(a, K, mask, X, Y, s, acc);
+                    } else if (bounce) {
+                        bounce_target<MODE>(K, mask, acc);
+                    } else if ((mask & (mask - 1)) == 0 && (kind == TSLB_BC_VELOCITY || kind == TSLB_BC_PRESSURE)) {
+                        mom_take(s);
+                        face_target<MODE>(a, K, m, dt, f, acc);
+                    } else {
+                        boundary_target<MODE, T, TAU, SOLID>(a, K, mask, X, Y, s, acc);
+                    }
+                }
+            }
+            // ---- x sums, y values ----
+            float dm = 0.f, dp = 0.f, upd = 0.f, dnd = 0.f;
+            if (COL && !zsolid) {
+                // phi differences along x and y (0 for a node that sends nothing)
+                dm = F::sub(sh.lo(pc), pc);
+                dp = F::sub(sh.hi(pc), pc);
+                const float* r = ring + (s & (RING - 1)) * RAREA + ri;
+                float pd = r[-RW], pu = r[RW];
+                if (!FAST && solid_bit(OUTD, nd.off, gz)) pd = 0.f;
+                if (!FAST && solid_bit(OUTU, nu.off, gz)) pu = 0.f;
+                upd = F::sub(pc, pu);
+                dnd = F::sub(pc, pd);
+            }
+            // recolouring sum_c (w_c / |c|) c.B over the neighbours, by class of |c|
+            float rB = 0.f, rE1 = 0.f, rE2 = 0.f, rZc = 0.f, rZs = 0.f;
+            constexpr float w1 = 16.f, w2 = 4.f * 0.70710678118654752f, w3 = 0.57735026918962576f;
+            if (COL && iface) {
+                auto sum = [&](float v) { return F::add(sh.lo(v), sh.hi(v)); };
+                rB = F::sub(sh.lo(K[K_C1]), sh.hi(K[K_C1]));
+                const float sy = sum(K[K_C2]), sz = sum(K[K_C3]);
+                rE1 = F::fma(0.25f * w2, sy, F::mul(0.25f * w1, K[K_C2]));
+                rE2 = F::fma(w3, sy, F::mul(w2, K[K_C2]));
+                rZc = F::fma(0.25f * w2, sz, F::mul(0.25f * w1, K[K_C3]));
+                rZs = F::fma(w3, sz, F::mul(w2, K[K_C3]));
+            }
+            if (COL) rest = K[K_C4];
+            // y values of one k: the sums at cy = 1 and -1 go to the rows above and below
+            auto send = [&](int k, V2 td, V2 sc, const YVal& ytd, const YVal& ysc) {
+                ktd[k] = td;
+                ksc[k] = sc;
+                ex[(0 * 3 + k) * NT + tid] = make_float4(ytd.p.x, ytd.p.y, ysc.p.x, ysc.p.y);
+                ex[(1 * 3 + k) * NT + tid] = make_float4(ytd.m.x, ytd.m.y, ysc.m.x, ysc.m.y);
+            };
+            {   // k = 0
+                const XSum j0 = xsum<3, COL, true>(K[K_0], K[K_X], K[K_XX], dm, dp, sh);
+                const XSum j1 = xsum<3, COL, false>(K[K_Y], K[K_XY], K[K_XXY], dm, dp, sh);
+                const XSum j2 = xsum<2, COL, false>(K[K_YY], K[K_XYY], 0.f, dm, dp, sh);
+                const YVal t = yval<3>(j0.td, j1.td, j2.td);
+                YVal c = yval<3>(j0.sc, j1.sc, j2.sc);
+                V2 cc = j0.sc;
+                if (COL) {
+                    // the receiver's phi difference; the x weights of the constant 1 sum to 6
+                    c.p.y = F::fma(upd, F::add(t.p.x, 6.f), c.p.y);
+                    c.m.y = F::fma(dnd, F::add(t.m.x, 6.f), c.m.y);
+                    if (iface) {
+                        const float h = F::mul(0.25f * w2, rB);
+                        cc.y = F::add(cc.y, rB);
+                        c.p.y = F::add(c.p.y, F::add(h, rE1));
+                        c.m.y = F::add(c.m.y, F::sub(h, rE1));
+                    }
+                }
+                if (PF) {
+                    // phase field g (D3Q7): axis directions and the rest population (q = 0:
+                    // p0g phi = 2 G0), in units of 1/4 and 1/16 like the sums beside them
+                    const float g0 = K[K_C0];
+                    const float sx = F::add(sh.lo(F::add(g0, K[K_C1])), sh.hi(F::sub(g0, K[K_C1])));
+                    cc.y = F::mul(0.0625f, F::fma(2.f, g0, sx));
+                    c.p.y = F::mul(0.25f, F::add(g0, K[K_C2]));
+                    c.m.y = F::mul(0.25f, F::sub(g0, K[K_C2]));
+                    rest = g0;
+                    gzf = K[K_C3];
+                }
+                send(0, j0.td, cc, t, c);
+            }
+            {   // k = 1
+                const XSum j0 = xsum<3, COL, false>(K[K_Z], K[K_XZ], K[K_XXZ], dm, dp, sh);
+                const XSum j1 = xsum<2, COL, false>(K[K_YZ], K[K_XYZ], 0.f, dm, dp, sh);
+                const XSum j2 = xsum<1, COL, false>(K[K_YYZ], 0.f, 0.f, dm, dp, sh);
+                const YVal t = yval<3>(j0.td, j1.td, j2.td);
+                YVal c = yval<3>(j0.sc, j1.sc, j2.sc);
+                V2 cc = j0.sc;
+                if (COL) {
+                    c.p.y = F::fma(upd, t.p.x, c.p.y);
+                    c.m.y = F::fma(dnd, t.m.x, c.m.y);
+                    if (iface) {
+                        cc.y = F::add(cc.y, rZc);
+                        c.p.y = F::add(c.p.y, rZs);
+                        c.m.y = F::add(c.m.y, rZs);
+                    }
+                }
+                send(1, j0.td, cc, t, c);
+            }
+            {   // k = 2
+                const XSum j0 = xsum<2, COL, false>(K[K_ZZ], K[K_XZZ], 0.f, dm, dp, sh);
+                const XSum j1 = xsum<1, COL, false>(K[K_YZZ], 0.f, 0.f, dm, dp, sh);
+                const YVal t = yval<2>(j0.td, j1.td, zero2);
+                YVal c = yval<2>(j0.sc, j1.sc, zero2);
+                V2 cc = j0.sc;
+                if (COL) {
+                    c.p.y = F::fma(upd, t.p.x, c.p.y);
+                    c.m.y = F::fma(dnd, t.m.x, c.m.y);
+                    if (iface) {
+                        // what k = 0 put into the planes s+-1 is taken out again
+                        const float h = F::mul(w3 - 0.25f * w2, rB), e = F::sub(rE2, rE1);
+                        cc.y = F::fma(0.25f * w2 - 1.f, rB, cc.y);
+                        c.p.y = F::add(c.p.y, F::add(h, e));
+                        c.m.y = F::add(c.m.y, F::sub(h, e));
+                    }
+                }
+                send(2, j0.td, cc, t, c);
             }
         }
         // phase field: candidates of the next source plane (its phi is staged)
-        if (MODE == TSLB_MODE_PHASEFIELD) {
+        if (PF) {
             if (more) list_candidates(s + 1);
-            else slot0 = slot1 = -1;
+            else cslot = -1;
         }
-        // VEC: all copies issued so far (moments of s+1, phi of s+2) land before the
-        // barrier, which also makes them visible for the next plane's coefficients
-        if (VEC) cp_async_wait<0>();
-        else cp_async_wait<1>();  // this thread's phi copies of plane s+2 have landed
+        if (PHI && !ASYNC && more) phi_store(s + 1 + RIM, ph);
+        cp_async_wait<1>();   // this thread's phi copies have landed
         __syncthreads();
-        // ---- 2. pull ----
-        if (active) {
-            const CNode Kc = cnode(coef, (ty + 1) * CW + (tx + 1));
-            float phm = 0.f, ph0 = 0.f, php = 0.f;
-            if (MODE == TSLB_MODE_COLOUR) {
-                // own-column phi of the target planes s-1 .. s+1
-                const int po = (ty + PHR) * SW + (tx + EPC);
-                phm = cvt_in<T>(phis[((s - 1) & (PRING - 1)) * PAREA + po], a, F_PHI);
-                ph0 = cvt_in<T>(phis[(s & (PRING - 1)) * PAREA + po], a, F_PHI);
-                php = cvt_in<T>(phis[((s + 1) & (PRING - 1)) * PAREA + po], a, F_PHI);
-            }
-            if (!zsolid) {
-                pull_row<MODE, -1>(Kc, accm, acc0, accp, phm, ph0, php);
-                pull_row<MODE, 0>(Kc, accm, acc0, accp, phm, ph0, php);
-                pull_row<MODE, 1>(Kc, accm, acc0, accp, phm, ph0, php);
-            }
-            // ---- 3. populations from behind non-periodic faces, target plane s ----
-            if (s >= z0 && s < z1) {
-                unsigned mask = colmask;
-                if (!zper && s == 0) mask |= 16u;
-                if (!zper && s == a.nz - 1) mask |= 32u;
-                const bool near_solid = SOLID && bit_at(a.near, (long long)s * plane + cn0.off);
-                if (mask || near_solid) boundary_target<MODE, T, TAU, SOLID>(a, Kc, mask, X, Y, s, acc0);
-            }
-            // ---- 4. target plane s-1 is complete ----
-            const int t = s - 1;
-            if (t >= z0 && t < z1) {
-                const float d = accm[A_RHO], rho = 1.f + d, inv = 1.f / rho;
-                const float u = accm[A_JX] * inv, v = accm[A_JY] * inv, w = accm[A_JZ] * inv;
-                const float d3 = d * (1.f / 3.f);
-                float o[NF];
-                o[F_D] = d;
-                o[F_U] = u; o[F_V] = v; o[F_W] = w;
-                o[F_XX] = accm[A_XX] - d3 - rho * u * u;
-                o[F_YY] = accm[A_YY] - d3 - rho * v * v;
-                o[F_ZZ] = accm[A_ZZ] - d3 - rho * w * w;
-                o[F_XY] = accm[A_XY] - rho * u * v;
-                o[F_XZ] = accm[A_XZ] - rho * u * w;
-                o[F_YZ] = accm[A_YZ] - rho * v * w;
-                // colour mode: phi_t + (colour increment) / rho
-                o[F_PHI] = MODE == TSLB_MODE_COLOUR ? fmaf(accm[A_COL], inv, phm) : accm[A_COL];
-                T* po = gout + (long long)t * plane + cn0.off;
-                if (SOLID && bit_at(a.solid, (long long)t * plane + cn0.off)) {
-                    // interior solid nodes keep their moments
-                    const T* pi = gin + (long long)t * plane + cn0.off;
+        if (!wtgt) return;
+        // ---- 3. y and z sums ----
+        V2 HA[3], HB[3], HM[3];
+        float H2[3];
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) po[f * a.N] = pi[f * a.N];
-                } else {
-                // single-component mode does not step phi (held at 1 in both buffers)
-                constexpr int nout = MODE == TSLB_MODE_SINGLE ? F_PHI : NF;
-                bool bad;
-                if constexpr (sizeof(T) == 2) {
-                    // 16-bit storage: two fields per conversion (store_pair16), stochastic
-                    // rounding seeded by the node (its index in the whole lattice) and the step
-                    const unsigned int hnode = sr_node((unsigned int)((t + a.zoff) * plane + cn0.off), sr_step);
-                    float vmax = 0.f;
-#pragma unroll
-                    for (int f = 0; f < nout; f += 2) {
-                        const int g = f + 1 < nout ? f + 1 : f;
-                        vmax = fmaxf(vmax, store_pair16<T>(po, a, f, g, o[f], o[g], a.sr, sr_field(hnode, f)));
-                    }
-                    // non-finite, or beyond the storage's range (NaN fails the comparison)
-                    bad = !(vmax <= Stor16Max<T>::value);
-                } else {
-                    float chk = 0.f;
-#pragma unroll
-                    for (int f = 0; f < nout; ++f) {
-                        po[f * a.N] = o[f];
-                        chk += o[f];
-                    }
-                    bad = !isfinite(chk);
-                }
-                if (bad) atomicOr(a.flags, 1u);
-                }
-            }
+        for (int k = 0; k < 3; ++k) {
+            // from the row below (cy = 1) and above (cy = -1)
+            const float4 lo = ex[(0 * 3 + k) * NT + max(tid - 32, lane)];
+            const float4 hi = ex[(1 * 3 + k) * NT + min(tid + 32, NT - 32 + lane)];
+            const V2 ltd = make_float2(lo.x, lo.y), htd = make_float2(hi.x, hi.y);
+            const V2 std_ = A::add(ltd, htd), ssc = A::add(make_float2(lo.z, lo.w), make_float2(hi.z, hi.w));
+            HA[k] = A::fma(A::c(4.f), ktd[k], std_);
+            HB[k] = A::fma(A::c(4.f), ksc[k], ssc);
+            HM[k] = A::sub(ltd, htd);
+            H2[k] = std_.x;
         }
-        // rotate the target slots
+        const V2 tA = A::add(HA[0], HA[2]), tB = A::add(HB[0], HB[2]), tM = A::add(HM[0], HM[2]);
+        const float t2 = F::add(H2[0], H2[2]);
+        const V2 pA = A::add(tA, HA[1]), mA = A::sub(tA, HA[1]), pM = A::add(tM, HM[1]), mM = A::sub(tM, HM[1]);
+        V2 pB = A::add(tB, HB[1]), mB = A::sub(tB, HB[1]);
+        const float p2 = F::add(t2, H2[1]), m2 = F::sub(t2, H2[1]);
+        const float pm_ = COL ? phi_of(s - 1) : 0.f;
+        if (COL) {
+            const float pn = phi_of(s + 1);
+            // the receiver's phi difference; the x and y weights of the constant 1 sum to 36
+            pB.y = F::fma(F::sub(pc, pn), F::add(pA.x, 36.f), pB.y);
+            mB.y = F::fma(F::sub(pc, pm_), F::add(mA.x, 36.f), mB.y);
+        }
+        if (PF) {
+            pB.y = F::add(rest, gzf);
+            mB.y = F::sub(rest, gzf);
+        }
+        // ---- target plane s-1 is complete ----
+        M0A = A::add(M0A, mA); M0B = A::add(M0B, mB); M0M = A::add(M0M, mM);
+        M02 = F::add(M02, m2);
+        M1A = A::sub(M1A, mA);
+        M1b = F::sub(M1b, mM.x);
+        M2 = F::add(M2, mA.x);
+        const int t = s - 1;
+        if (valid && t >= z0) {
+            constexpr float c216 = 1.f / 216.f;
+            const float d = F::mul(M0A.x, c216), rho = F::add(d, 1.f), inv = F::mul(__frcp_rn(rho), c216);
+            float o[NF];
+            o[F_D] = d;
+            const float u = o[F_U] = F::mul(M0A.y, inv), v = o[F_V] = F::mul(M0M.x, inv), w = o[F_W] = F::mul(M1A.x, inv);
+            const float ru = F::mul(-rho, u), rv = F::mul(-rho, v), rw = F::mul(-rho, w), d3 = F::mul(d, -1.f / 3.f);
+            o[F_XX] = F::fma(ru, u, F::fma(M0B.x, c216, d3));
+            o[F_YY] = F::fma(rv, v, F::fma(M02, c216, d3));
+            o[F_ZZ] = F::fma(rw, w, F::fma(M2, c216, d3));
+            o[F_XY] = F::fma(ru, v, F::mul(M0M.y, c216));
+            o[F_XZ] = F::fma(ru, w, F::mul(M1A.y, c216));
+            o[F_YZ] = F::fma(rv, w, F::mul(M1b, c216));
+            // colour mode: phi_t + (colour increment) / rho
+            o[F_PHI] = COL ? F::fma(M0B.y, inv, pm_) : M0B.y;
+            float chk = 0.f;
+            if (sizeof(T) == 4) {
 #pragma unroll
-        for (int i = 0; i < NACC; ++i) { accm[i] = acc0[i]; acc0[i] = accp[i]; accp[i] = 0.f; }
-        buf ^= 1;
+                for (int f = 0; f < (PHI ? NF : F_PHI); ++f) chk = F::add(chk, o[f]);
+            }
+            store_target<MODE, T, SOLID>(a, (unsigned)t * plane + n0.off, plane, sr_step, o, chk);
+        }
+        // ---- rotate: target s becomes the one to complete, s+1 opens ----
+        M1A = UA; M1b = UM.x; M2 = UA.x;
+        M0A = A::fma(A::c(4.f), HA[0], UA);
+        M0B = A::fma(A::c(4.f), HB[0], UB);
+        M0M = A::fma(A::c(4.f), HM[0], UM);
+        M02 = F::fma(4.f, H2[0], U02);
+        UA = pA; UB = pB; UM = pM; U02 = p2;
+        if (COL) M0A.x = F::fma(216.f, rest, M0A.x);   // rest population: f_0 += delta0
+        if (!FAST && near) {
+            auto add = [&](float& v, int i) { v = F::fma(216.f, bnd[i * NT + tid], v); };
+            add(M0A.x, A_RHO); add(M0A.y, A_JX); add(M0B.x, A_XX); add(M0M.x, A_JY); add(M0M.y, A_XY); add(M02, A_YY);
+            add(M1A.x, A_JZ); add(M1A.y, A_XZ); add(M1b, A_YZ); add(M2, A_ZZ);
+            if (COL) add(M0B.y, A_COL);
+            if (PF) M0B.y = F::add(M0B.y, bnd[A_COL * NT + tid]);
+        }
+    };
+    const int f0 = max(z0 - 1, 1), f1 = min(z1, a.nz - 2 - RIM);
+    for (int s = z0 - 1; s <= z1;) {
+        if (inner && s >= f0 && s <= f1) {
+#pragma unroll 1
+            for (; s <= f1; ++s) iterate(std::true_type{}, s);
+        } else {
+            iterate(std::false_type{}, s);
+            ++s;
+        }
     }
     cp_async_wait<0>();
 }
 
-template <int MODE, bool VEC, class T, bool TAU = false, bool SOLID = false>
-__global__ void __launch_bounds__(NTHR, 2) step_kernel(const StepArgs a) {
-    step_block<MODE, VEC, T, TAU, SOLID>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+// Blocks of consecutive index work on tiles next to each other in x, at the
+// same planes, so that the rows and memory sectors they share are read from
+// DRAM once.  zchunk > 0: every block takes one chunk of zchunk planes of a
+// tile.  zchunk = 0: the tiles of one x position, each with all its target
+// planes, are a sequence of planes; grid / tx blocks take equal shares of it,
+// in one piece or, across the end of a tile, in several.
+template <int MODE, class T, int W, bool TAU = false, bool SOLID = false>
+__global__ void __launch_bounds__(32 * W, BIGW / W) step_kernel(const __grid_constant__ StepArgs a) {
+    const int planes = a.zt1 - a.zt0, tx = a.xwrap ? 1 : (a.nx + LXV - 1) / LXV, ty = (a.ny + a.th - 1) / a.th;
+    const int bx = blockIdx.x % tx, b = blockIdx.x / tx;
+    int p, end;   // the block's part of the sequence
+    if (a.zchunk > 0) {
+        const int first = b % ty * planes, z = b / ty * a.zchunk;
+        p = first + z;
+        end = first + min(z + a.zchunk, planes);
+    } else {
+        const long long total = (long long)ty * planes, n = gridDim.x / tx;
+        p = (int)(total * b / n);
+        end = (int)(total * (b + 1) / n);
+    }
+    while (p < end) {
+        const int by = p / planes, z = p % planes, n = min(end - p, planes - z);
+        step_block<MODE, T, W, TAU, SOLID>(a, bx, by, a.zt0 + z, a.zt0 + z + n);
+        p += n;
+        if (p < end) __syncthreads();
+    }
 }
 
 // Work item of the ensemble kernel: lattice, tile column, z chunk.
@@ -1065,13 +1240,13 @@ struct WorkItem {
 // whichever block asks next (a work counter), so a grid smaller than the
 // list balances items of uneven length.  The lattice's arguments are staged
 // in shared memory when the block moves to a new lattice.  All lattices
-// share MODE, VEC and T.  step[0] is the step counter that seeds the
+// share MODE and T.  step[0] is the step counter that seeds the
 // stochastic rounding (every member's arguments point at it), step[1] a
 // ticket and step[2] the work counter: the last block of the launch to
 // finish, after every block has read the step and taken its last item,
 // advances the step and clears the other two for the next launch.
-template <int MODE, bool VEC, class T>
-__global__ void __launch_bounds__(NTHR, 2) ensemble_kernel(const StepArgs* __restrict__ args,
+template <int MODE, class T>
+__global__ void __launch_bounds__(32 * SMALLW, BIGW / SMALLW) ensemble_kernel(const StepArgs* __restrict__ args,
                                                           const WorkItem* __restrict__ work, int nwork,
                                                           unsigned int* step) {
     __shared__ StepArgs sa;
@@ -1084,11 +1259,11 @@ __global__ void __launch_bounds__(NTHR, 2) ensemble_kernel(const StepArgs* __res
             const int words = (int)(sizeof(StepArgs) / sizeof(int));
             const int* src = reinterpret_cast<const int*>(args + w.dom);
             int* dst = reinterpret_cast<int*>(&sa);
-            for (int i = threadIdx.y * TX + threadIdx.x; i < words; i += NTHR) dst[i] = src[i];
+            for (int i = threadIdx.y * 32 + threadIdx.x; i < words; i += 32 * SMALLW) dst[i] = src[i];
             __syncthreads();
             cur = w.dom;
         }
-        step_block<MODE, VEC, T, false, false, MODE != TSLB_MODE_PHASEFIELD>(sa, w.bx, w.by, w.bz);
+        step_block<MODE, T, SMALLW>(sa, w.bx, w.by, sa.zt0 + w.bz * sa.zchunk, min(sa.zt0 + (w.bz + 1) * sa.zchunk, sa.zt1));
         __syncthreads();
         // every thread has read `next` (it was read before this item's barriers)
         if (step) {
