@@ -27,8 +27,8 @@ struct tslb_ctx {
     float* nrm = nullptr;                  // 3 fields
     float* inlet[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     unsigned int* flags = nullptr;
-    // FP64 diagnostics: red_blocks x RED_PARTS per-block partials, then the
-    // RED_PARTS results and the last-block ticket; red_host is pinned
+    // FP64 diagnostics: RED_PARTS x red_blocks per-block partials, then the
+    // last-block ticket; red_host is pinned, and the kernel writes the results there
     double* red = nullptr;
     double* red_host = nullptr;
     double* red_ring = nullptr;            // tslb_reduce_async results (pinned, TSLB_REDUCE_QUEUE slots)
@@ -69,8 +69,8 @@ struct tslb_ctx {
 namespace tslb_internal {
 // record msg as the context's (or, for ctx == NULL, the creation) error; returns code
 int fail(tslb_ctx* c, int code, const std::string& msg);
-// FP32 view of the current state (converted through io for bf16/fp16 storage)
-int fp32_view(tslb_ctx* c, const float** out);
+// FP32 view of the current state (bf16/fp16 storage: the fields of these bits, converted into io)
+int fp32_view(tslb_ctx* c, const float** out, unsigned fields = ~0u);
 // allocate the per-node tau correction buffer (zeroed) if absent
 int ensure_dtau(tslb_ctx* c);
 // closure.cu: refresh c->dtau from the attached closure before a step
