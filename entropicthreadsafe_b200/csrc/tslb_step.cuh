@@ -381,7 +381,10 @@ constexpr int ROWE = 40, MROW = ROWE * 4;   // elements, and bytes kept for a ro
 template <int MODE, int W>
 struct Smem {
     static constexpr int NT = 32 * W;
-    static constexpr int RAREA = ROWE * (W + 2 * phi_rim(MODE));
+    // (a plane of the ring is 12 banks past the one before: the curvature's lanes
+    // read three planes at once)
+    static constexpr int RAREA = (ROWE * (W + 2 * phi_rim(MODE)) + 31) / 32 * 32 + 12;
+    static_assert(RAREA % 4 == 0, "16-byte rows");
     static constexpr int exch = 0;
     static constexpr int mom = exch + 2 * 2 * 3 * NT * 16;
     static constexpr int dt = mom + 2 * NMOM * W * MROW;
@@ -422,18 +425,7 @@ __device__ __forceinline__ void grad_v(LD P, typename Ar::V g[3]) {
     g[1] = Ar::fma(c3, y3, Ar::fma(c2, y2, Ar::mul(c1, y1)));
     g[2] = Ar::fma(c3, z3, Ar::fma(c2, z2, Ar::mul(c1, z1)));
 }
-// one node; pm, p0, pp point at it in planes z-1, z, z+1 (row pitch SWv).
-template <int SWv>
-__device__ __forceinline__ void grad_smem(const float* pm, const float* p0, const float* pp, float g[3]) {
-    grad_v<Ar1>([&](int dz, int dx, int dy) {
-        const float* pl = dz < 0 ? pm : dz > 0 ? pp : p0;
-        return pl[dy * SWv + dx];
-    }, g);
-}
-
-// Phase-field interface normal n = g / (|g| + 1e-9) from the staged phi
-// planes (ring slots of plane z and its neighbours), at staged offset pi
-// (recursive_2c_TSLB3D.f90:555-571).
+// Phase-field interface normal (recursive_2c_TSLB3D.f90:555-571)
 // n = g / (|g| + 1e-9) of one node (Ar1) or two (Ar2), operation by operation
 template <class Ar>
 __device__ __forceinline__ void normalize_v(typename Ar::V n[3]) {
@@ -446,15 +438,6 @@ template <class Ar>
 __device__ __forceinline__ typename Ar::V pf_indicator(typename Ar::V phi, const typename Ar::V n[3]) {
     const typename Ar::V nn = Ar::fma(n[2], n[2], Ar::fma(n[1], n[1], Ar::mul(n[0], n[0])));
     return Ar::mul(Ar::mul(phi, Ar::sub(Ar::c(1.f), phi)), nn);
-}
-
-template <int SWv>
-__device__ __forceinline__ void pf_normal(const float* ring, int parea, int z, int pi, float n[3]) {
-    const float* p0 = ring + (z & (RING - 1)) * parea + pi;
-    const float* pm = ring + ((z - 1) & (RING - 1)) * parea + pi;
-    const float* pp = ring + ((z + 1) & (RING - 1)) * parea + pi;
-    grad_smem<SWv>(pm, p0, pp, n);
-    normalize_v<Ar1>(n);
 }
 
 struct XYNode {
@@ -473,37 +456,51 @@ __device__ __forceinline__ XYNode xy_node(const StepArgs& a, int gx, int gy, boo
     return n;
 }
 
-// Phase-field curvature -div n of one coefficient node, computed by a whole
-// warp: the isotropic stencil over the node's 26 neighbours
-// (recursive_2c_TSLB3D.f90:617-627), each neighbour's normal recomputed from
-// the staged phi (pf_normal); a neighbour behind a non-periodic face, or an
-// interior solid one, has n = 0.  Lane j < 26 computes neighbour j and a
-// butterfly sums the 26 terms; every lane returns the sum.  z is the source
-// plane (ring index), gz its lattice plane, pi the node's staged offset and
-// (gx, gy) its lattice coordinates (may lie beyond a periodic face).
-template <int SWv, bool SOLID>
-__device__ float node_curvature(const float* ring, int parea, int z, int pi, int gx, int gy, int gz, const StepArgs& a,
-                                bool xper, bool yper, bool zper) {
-    const int lane = threadIdx.x;
-    const int j = lane < 13 ? lane : lane + 1;   // 3 x 3 x 3 index of the neighbour, the centre (13) skipped
-    const int dx = j % 3 - 1, dy = (j / 3) % 3 - 1, dz = j / 9 - 1;
-    const int xn = gx + dx, yn = gy + dy, zn = gz + dz;
-    bool ok = lane < 26 && (zper || (zn >= 0 && zn < a.nz)) && (xper || (xn >= 0 && xn < a.nx)) &&
-              (yper || (yn >= 0 && yn < a.ny));
-    if (SOLID && ok) ok = !bit_at(a.solid, nidx(a, wrapi(xn, a.nx), wrapi(yn, a.ny), wrapi(zn, a.nz)));
-    float t = 0.f;
-    if (ok) {
-        float n[3];
-        pf_normal<SWv>(ring, parea, z + dz, pi + dy * SWv + dx, n);
-        t = __fmul_rn(wclass(dx * dx + dy * dy + dz * dz),
-                      __fmaf_rn((float)dz, n[2], __fmaf_rn((float)dy, n[1], __fmul_rn((float)dx, n[0]))));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
-    return __fmul_rn(-3.f, t);
-}
-
 using V2 = Ar2::V;
+
+// Phase-field curvature -div n of two coefficient nodes (one per lane of the
+// pairs), computed by a whole warp: the isotropic stencil over the nodes' 26
+// neighbours (recursive_2c_TSLB3D.f90:617-627), each neighbour's normal
+// recomputed from the staged phi; a neighbour behind a non-periodic face, or an
+// interior solid one, has n = 0.  Lane j < 26 computes neighbour j of both
+// and a butterfly sums the 26 terms; every lane returns the sums.  z is the
+// source plane (ring index), gz its lattice plane, pi the nodes' staged offsets
+// and (gx, gy) their lattice coordinates (may lie beyond a periodic face).
+// What bounds it is the latency of one node's chain (loads, square root,
+// reciprocal, butterfly), so two nodes go through it together.
+template <int SWv, bool SOLID>
+__device__ __forceinline__ V2 node_curvature(const float* ring, int parea, int z, const int pi[2], const int gx[2],
+                                             const int gy[2], int gz, const StepArgs& a, bool xper, bool yper, bool zper) {
+    using A = Ar2;
+    const int lane = threadIdx.x;
+    const int j = lane < 13 ? lane : min(lane + 1, 26);   // 3 x 3 x 3 index of the neighbour, the centre (13) skipped
+    const int dx = j % 3 - 1, dy = (j / 3) % 3 - 1, dz = j / 9 - 1;
+    bool ok[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int xn = gx[k] + dx, yn = gy[k] + dy, zn = gz + dz;
+        ok[k] = lane < 26 && (zper || (zn >= 0 && zn < a.nz)) && (xper || (xn >= 0 && xn < a.nx)) &&
+                (yper || (yn >= 0 && yn < a.ny));
+        if (SOLID && ok[k]) ok[k] = !bit_at(a.solid, nidx(a, wrapi(xn, a.nx), wrapi(yn, a.ny), wrapi(zn, a.nz)));
+    }
+    const int o = dy * SWv + dx;
+    const float *p0 = ring + ((z + dz) & (RING - 1)) * parea + o, *pm = ring + ((z + dz - 1) & (RING - 1)) * parea + o,
+                *pp = ring + ((z + dz + 1) & (RING - 1)) * parea + o;
+    V2 n[3];
+    grad_v<A>([&](int ez, int ex, int ey) {
+        const float* p = (ez < 0 ? pm : ez > 0 ? pp : p0) + ey * SWv + ex;
+        return make_float2(p[pi[0]], p[pi[1]]);
+    }, n);
+    normalize_v<A>(n);
+    V2 t = A::mul(A::c(wclass(dx * dx + dy * dy + dz * dz)),
+                  A::fma(A::c((float)dz), n[2], A::fma(A::c((float)dy), n[1], A::mul(A::c((float)dx), n[0]))));
+    if (!ok[0]) t.x = 0.f;
+    if (!ok[1]) t.y = 0.f;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1)
+        t = A::add(t, make_float2(__shfl_xor_sync(0xffffffffu, t.x, h), __shfl_xor_sync(0xffffffffu, t.y, h)));
+    return A::mul(A::c(-3.f), t);
+}
 
 // The value of the node at x - 1 (lo) and x + 1 (hi): the neighbouring lanes', or
 // with the whole periodic axis in a warp any two lanes'.
@@ -917,7 +914,6 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         // ---- 0. moments of the next plane, phi of the plane after the ring's last ----
         cp_async_wait<0>();
         __syncwarp();   // the warp's copies of the moments of plane s have landed
-        if (wact) mom_take(s);
         PhiRow ph;
         if (more) load_ahead(fast, s + 1, s + 1 + RIM, wact, ph);
         // ---- curvatures of this plane's candidates, warp w taking entries w, w + nw, ...
@@ -926,12 +922,20 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         if (PF) {
             const int cnt = cq_n[s & 1];
             if (cnt > 0) {
-                for (int e = wy; e < cnt; e += W) {
-                    const int ci = cq_list[(s & 1) * NT + e];
-                    const int cx = ci & 31, cy = ci >> 5;
-                    const float k = node_curvature<RW, SOLID>(ring, RAREA, s, (cy + RIM) * RW + rx + cx + RIM, X0 + cx,
-                                                              y0 - 1 + cy, gz, a, xper, yper, zper);
-                    if (lane == 0) cq_curv[e] = k;
+                for (int e = wy; e < cnt; e += 2 * W) {
+                    int pi[2], gx2[2], gy2[2];
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {   // (an odd last entry twice)
+                        const int ci = cq_list[(s & 1) * NT + (e + k * W < cnt ? e + k * W : e)];
+                        gx2[k] = X0 + (ci & 31);
+                        gy2[k] = y0 - 1 + (ci >> 5);
+                        pi[k] = ((ci >> 5) + RIM) * RW + rx + (ci & 31) + RIM;
+                    }
+                    const V2 k2 = node_curvature<RW, SOLID>(ring, RAREA, s, pi, gx2, gy2, gz, a, xper, yper, zper);
+                    if (lane == 0) {
+                        cq_curv[e] = k2.x;
+                        if (e + W < cnt) cq_curv[e + W] = k2.y;
+                    }
                 }
                 __syncthreads();
                 // every thread has read cnt; the next entries of this parity come after the plane barrier
@@ -945,6 +949,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         if (wact) {
             // ---- 1. coefficients ----
             float g[3], K[NCOEF];
+            mom_take(s);
             if (PHI) {
                 const Sten q = stencil(s + 1);
                 constexpr float k72 = 1.f / 72.f;
