@@ -54,6 +54,7 @@ static thread_local std::string g_closure_create_error;
 namespace {
 
 constexpr int TRAIN_SMEM = 104 * 1024;   // caps residency at 2 CTAs/SM (256 TMEM columns each)
+constexpr int IMG16 = (int)(sizeof(Image) / 16);   // the image in 16-byte words
 constexpr int OFF_ACT = IMG_BYTES, OFF_DZ = IMG_BYTES + ACT_BYTES;
 constexpr int OFF_MISC_TRAIN = OFF_DZ + DZ_BYTES, OFF_MISC_INFER = OFF_ACT + Act<NCH_INFER>::BYTES;
 // image + 10-chunk ACT + barrier words: at most 7 CTAs/SM (64 TMEM columns each)
@@ -99,7 +100,10 @@ __global__ void image_kernel(const float* __restrict__ params, Image* img) {
     }
 }
 
-// Shared-memory prologue of the MLP kernels: image copy, mbarrier, TMEM.
+// Shared-memory prologue of the MLP kernels: mbarrier, TMEM, the image copy.
+// The training kernel is launched while the optimiser of the step before may
+// still be writing the image (train_pass): `before` runs first, then the
+// kernel waits for that step, and only then is the image read.
 struct Smem {
     Image* im;
     uint4* act;
@@ -110,7 +114,9 @@ struct Smem {
     float* red;
 };
 
-__device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int off_misc, bool train, uint32_t ncols) {
+template <class Before>
+__device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int off_misc, bool train, uint32_t ncols,
+                                           Before before) {
     Smem S;
     S.im = reinterpret_cast<Image*>(sm);
     S.act = reinterpret_cast<uint4*>(sm + OFF_ACT);
@@ -120,9 +126,6 @@ __device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int o
     S.abort_s = reinterpret_cast<int*>(sm + off_misc + 12);
     S.red = reinterpret_cast<float*>(sm + off_misc + 64);
     const int tid = threadIdx.x;
-    const uint4* src = reinterpret_cast<const uint4*>(gimg);
-    uint4* dst = reinterpret_cast<uint4*>(sm);
-    for (int i = tid; i < (int)(sizeof(Image) / 16); i += blockDim.x) dst[i] = src[i];
     if (train) {
         // constant chunks of ACT: a 1 in the first column of chunk 10, zeros in chunk 11
         const float one[8] = {1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -134,6 +137,16 @@ __device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int o
         *S.abort_s = 0;
     }
     if ((tid >> 5) == 0) tc::tmem_alloc(S.tslot, ncols);
+    before();
+    if (train) {
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+    }
+    const uint4* src = reinterpret_cast<const uint4*>(gimg);
+    uint4* dst = reinterpret_cast<uint4*>(sm);
+#pragma unroll
+    for (int k = 0; k < (IMG16 + TILE - 1) / TILE; ++k)
+        if (tid + k * TILE < IMG16) dst[tid + k * TILE] = src[tid + k * TILE];
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -244,7 +257,7 @@ template <class Src>
 __global__ void __launch_bounds__(TILE, 6) infer_kernel(const Image* __restrict__ gimg, Src src, long long n,
                                                         unsigned int* gflag) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    Smem S = smem_setup(sm, gimg, OFF_MISC_INFER, false, 64);
+    Smem S = smem_setup(sm, gimg, OFF_MISC_INFER, false, 64, [] {});
     const uint32_t tb = *S.tslot;
     const Image& im = *S.im;
     const int tid = threadIdx.x;
@@ -309,11 +322,43 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
+// A partial gradient keeps the two weight matrices transposed (inputs x
+// units), so that the lanes of the training kernel, which own units, store
+// neighbouring words; parameter of a position below NPARAM.
+__device__ __forceinline__ int param_of(int pos) {
+    if (pos < P_B1) return (pos % NH) * KIN + pos / NH;
+    if (pos >= P_W2 && pos < P_B2) return P_W2 + ((pos - P_W2) % NH) * NH + (pos - P_W2) / NH;
+    return pos;
+}
+
 // Forward + backward of the batch; each CTA writes its partial gradient
 // (summed over its tiles in tensor memory) and loss to a.partial.
+// A batch of 16,384 is one tile per CTA: the time is one chain of a gather,
+// four tensor-core steps with their epilogues, and the partial's store, not
+// throughput.  So the draw and the gather of a tile run before the image is
+// waited for (first tile) or behind the tile before, the partials are stored
+// a warp's 128 bytes at a time, and the 64 sums over a warp's rows halve
+// their values with their lanes (62 shuffles; 320 one by one).  A training
+// step of that batch, both kernels: 26.1 us before, 10.8 us now.
 __global__ void __launch_bounds__(TILE, 1) train_kernel(const TrainArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    Smem S = smem_setup(sm, a.img, OFF_MISC_TRAIN, true, 256);
+    struct Row {
+        float f[NFEAT], tg, wg;
+    } row;
+    const long long ntiles = (a.nrows + TILE - 1) / TILE;
+    auto load_row = [&](long long t) {
+        const long long slot = t * TILE + threadIdx.x;
+        const bool valid = slot < a.nrows;
+        long long idx = slot;
+        if (a.random)
+            idx = (long long)(mix64(a.seed * 0x100000001B3ull ^ ((unsigned long long)a.step << 40) ^ (unsigned long long)slot) %
+                              (unsigned long long)a.ndata);
+#pragma unroll
+        for (int k = 0; k < NFEAT; ++k) row.f[k] = valid ? a.feat[idx * NFEAT + k] : 0.f;
+        row.tg = valid ? a.tgt[idx] : 0.f;
+        row.wg = valid ? a.wgt[idx] : 0.f;
+    };
+    Smem S = smem_setup(sm, a.img, OFF_MISC_TRAIN, true, 256, [&] { load_row(blockIdx.x); });
     const uint32_t tb = *S.tslot;
     const Image& im = *S.im;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -325,19 +370,12 @@ __global__ void __launch_bounds__(TILE, 1) train_kernel(const TrainArgs a) {
     for (int j = 0; j < NH; ++j) dw3[j] = 0.f;
     float db3 = 0.f, lsum = 0.f;
     bool first = true;
-    const long long ntiles = (a.nrows + TILE - 1) / TILE;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const long long slot = t * TILE + tid;
         const bool valid = slot < a.nrows;
-        long long idx = slot;
-        if (a.random)
-            idx = (long long)(mix64(a.seed * 0x100000001B3ull ^ ((unsigned long long)a.step << 40) ^ (unsigned long long)slot) %
-                              (unsigned long long)a.ndata);
-        float f[NFEAT], tg = 0.f, wg = 0.f;
-#pragma unroll
-        for (int k = 0; k < NFEAT; ++k) f[k] = valid ? a.feat[idx * NFEAT + k] : 0.f;
-        if (valid) { tg = a.tgt[idx]; wg = a.wgt[idx]; }
-        put_x(S.act, tid, f, im, valid);
+        const float tg = row.tg, wg = row.wg;
+        put_x(S.act, tid, row.f, im, valid);
+        if (t + gridDim.x < ntiles) load_row(t + gridDim.x);
         sync_for_mma();
         if (tid == 0) {
             tc::fence_after_sync();
@@ -381,7 +419,7 @@ __global__ void __launch_bounds__(TILE, 1) train_kernel(const TrainArgs a) {
     }
     float* part = a.partial + (size_t)blockIdx.x * PSTRIDE;
     // weight and bias gradients of the two hidden layers from tensor memory
-    const int row = 32 * warp + lane;
+    const int unit = 32 * warp + lane;
     const bool have = !first && *S.abort_s == 0;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
@@ -394,23 +432,38 @@ __global__ void __launch_bounds__(TILE, 1) train_kernel(const TrainArgs a) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
             const int col = 32 * q + j;
-            if (row < NH) {
-                if (col < NH) part[P_W2 + row * NH + col] = d[j];
-                else if (col == 80) part[P_B2 + row] = d[j];
+            if (unit < NH) {
+                if (col < NH) part[P_W2 + col * NH + unit] = d[j];
+                else if (col == 80) part[P_B2 + unit] = d[j];
             } else {
-                const int u = row - NH;
-                if (col >= 64 && col < 80) part[P_W1 + u * KIN + (col - 64)] = d[j];
-                else if (col == 80) part[P_B1 + u] = d[j];
+                if (col >= 64 && col < 80) part[P_W1 + (col - 64) * NH + unit - NH] = d[j];
+                else if (col == 80) part[P_B1 + unit - NH] = d[j];
             }
         }
     }
-    // output-layer gradient and loss: block sums
+    // output-layer gradient and loss: block sums.  Lanes that differ in bit o
+    // send each other the half of the values that the other keeps; values
+    // 2 lane and 2 lane + 1 are left.
 #pragma unroll
-    for (int j = 0; j < NH + 2; ++j) {
-        float v = j < NH ? dw3[j] : (j == NH ? db3 : lsum);
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) S.red[warp * (NH + 2) + j] = v;
+        for (int j = 0; j < 2 * o; ++j) {
+            const float send = up ? dw3[j] : dw3[j + 2 * o];
+            dw3[j] = (up ? dw3[j + 2 * o] : dw3[j]) + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        db3 += __shfl_xor_sync(0xffffffffu, db3, o);
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    }
+    float* red = S.red + warp * (NH + 2);
+    red[2 * lane] = dw3[0];
+    red[2 * lane + 1] = dw3[1];
+    if (lane == 0) {
+        red[NH] = db3;
+        red[NH + 1] = lsum;
     }
     __syncthreads();
     if (tid < NH + 2) {
@@ -423,6 +476,11 @@ __global__ void __launch_bounds__(TILE, 1) train_kernel(const TrainArgs a) {
 // Sum the CTAs' partials in a fixed order; gradient mode writes the
 // gradient, training mode takes one Adam step on the master parameters and
 // rewrites their image.
+// A block takes 32 positions (a partial's 128-byte line), warp w of it the
+// partials w, w + 8, ..., and the first warp adds the eight sums and steps:
+// one thread a parameter over all partials was a chain of 128 loads in 21
+// blocks.
+constexpr int ADAM_WARPS = 8, ADAM_BLOCKS = (NPARAM_PAD + 1 + 31) / 32;   // positions up to the loss
 struct AdamArgs {
     const float* partial;
     int nctas;
@@ -435,26 +493,41 @@ struct AdamArgs {
     float* grad_out;      // gradient mode when non-null
     float* loss_out;
 };
-__global__ void adam_kernel(const AdamArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0 && a.loss_out) {
-        float l = 0.f;
-        for (int c = 0; c < a.nctas; ++c) l += a.partial[(size_t)c * PSTRIDE + NPARAM_PAD];
-        *a.loss_out = l;
+__global__ void __launch_bounds__(32 * ADAM_WARPS) adam_kernel(const AdamArgs a) {
+    __shared__ float sums[ADAM_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pos = blockIdx.x * 32 + lane;
+    const bool isloss = pos == NPARAM_PAD;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int p = pos < NPARAM ? param_of(pos) : 0;
+    float m = 0.f, v = 0.f, w = 0.f, g = 0.f;
+    if (warp == 0 && pos < NPARAM && !a.grad_out) {
+        m = a.m[p];
+        v = a.v[p];
+        w = a.params[p];
     }
-    if (p >= NPARAM) return;
-    float g = 0.f;
-    for (int c = 0; c < a.nctas; ++c) g += a.partial[(size_t)c * PSTRIDE + p];
+    if (pos < NPARAM || isloss) {
+#pragma unroll 16
+        for (int c = warp; c < a.nctas; c += ADAM_WARPS) g += a.partial[(size_t)c * PSTRIDE + pos];
+    }
+    sums[warp][lane] = g;
+    __syncthreads();
+    if (warp > 0) return;
+#pragma unroll
+    for (int k = 1; k < ADAM_WARPS; ++k) g += sums[k][lane];
+    if (isloss && a.loss_out) *a.loss_out = g;
+    if (pos >= NPARAM) return;
     if (p < P_B1 && (p % KIN) >= NFEAT) g = 0.f;   // padding inputs
     if (a.grad_out) {
         a.grad_out[p] = g;
         return;
     }
-    const float m = a.b1 * a.m[p] + (1.f - a.b1) * g;
-    const float v = a.b2 * a.v[p] + (1.f - a.b2) * g * g;
+    m = a.b1 * m + (1.f - a.b1) * g;
+    v = a.b2 * v + (1.f - a.b2) * g * g;
     a.m[p] = m;
     a.v[p] = v;
-    float w = a.params[p] - a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
+    w -= a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
     if (p < P_B1 && (p % KIN) >= NFEAT) w = 0.f;
     a.params[p] = w;
     __nv_bfloat16* w1 = reinterpret_cast<__nv_bfloat16*>(a.img->w1);
@@ -691,8 +764,22 @@ int train_pass(tslb_closure* c, const float* feat, const float* tgt, const float
     a.ndata = ndata; a.nrows = nrows; a.random = random; a.seed = seed; a.step = step;
     a.inv_batch = 1.0f / (float)nrows;
     a.partial = c->partial; a.flags = c->flags;
-    train_kernel<<<grid, TILE, TRAIN_SMEM, c->stream>>>(a);
-    CL_TRY(c, cudaGetLastError());
+    // The optimiser starts under the training kernel and a later step's
+    // training kernel under the optimiser; each waits on the device for the
+    // whole grid before it before it touches what that grid writes (partials,
+    // image).  The first kernel of a call follows in plain stream order: the
+    // samples it reads ahead of its wait may have been written just before.
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(TILE);
+    cfg.dynamicSmemBytes = TRAIN_SMEM;
+    cfg.stream = c->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = step > 0 ? 1 : 0;
+    CL_TRY(c, cudaLaunchKernelEx(&cfg, train_kernel, a));
     AdamArgs d;
     d.partial = c->partial; d.nctas = grid;
     d.params = c->params; d.m = c->adam_m; d.v = c->adam_v; d.img = c->img;
@@ -701,8 +788,11 @@ int train_pass(tslb_closure* c, const float* feat, const float* tgt, const float
     d.bc1 = 1.0f - std::pow(0.9f, (float)std::max<long long>(c->adam_t, 1));
     d.bc2 = 1.0f - std::pow(0.999f, (float)std::max<long long>(c->adam_t, 1));
     d.grad_out = grad_out; d.loss_out = loss_out;
-    adam_kernel<<<(NPARAM + 255) / 256, 256, 0, c->stream>>>(d);
-    CL_TRY(c, cudaGetLastError());
+    cfg.gridDim = dim3(ADAM_BLOCKS);
+    cfg.blockDim = dim3(32 * ADAM_WARPS);
+    cfg.dynamicSmemBytes = 0;
+    cfg.numAttrs = 1;
+    CL_TRY(c, cudaLaunchKernelEx(&cfg, adam_kernel, d));
     return TSLB_OK;
 }
 
