@@ -7,8 +7,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
+#include <map>
 #include <mutex>
 #include <new>
+#include <queue>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -1723,7 +1726,7 @@ struct tslb_ensemble {
     StepArgs* d_args[2] = {nullptr, nullptr};  // per step parity: member args
     WorkItem* d_work = nullptr;
     int nwork = 0;
-    int zchunk = 16;
+    int zchunk = 16;                   // most target planes of an item
     int grid = 0;                      // 0: one block per work item
     int sms = 148;
     int parity = 0;                    // steps taken mod 2 since the last args upload
@@ -1763,7 +1766,7 @@ int ens_build(tslb_ensemble* e) {
     std::vector<StepArgs> args[2];
     for (size_t d = 0; d < e->m.size(); ++d) {
         tslb_ctx* c = e->m[d];
-        c->zchunk = std::min(e->zchunk, c->nz);
+        c->zchunk = even_rows(c->nz, e->zchunk);
         c->th = even_rows(c->ny, SMALLW - 2);
         const StepArgs ca = make_args(c, nullptr, nullptr);
         const int gx = tslb_launch::tiles_x(ca), gy = tslb_launch::tiles_y(ca), gz = (c->nz + c->zchunk - 1) / c->zchunk;
@@ -1800,6 +1803,49 @@ int ens_build(tslb_ensemble* e) {
     }
     e->parity = 0;
     return TSLB_OK;
+}
+
+// The z chunk with the least estimated time, until a tuning or
+// tslb_ensemble_set_launch sets one.  An item costs its planes and about 3
+// more (two source planes outside its targets, its start), so long items are
+// cheap, but few of them leave blocks idle at the end of a step: the items
+// go, longest first, to the block that is free first.  48 droplets of 72 x 32^2
+// to 104 x 96^2 nodes: 16-plane chunks 1001 us a step, whole columns (chosen)
+// 887 us; 4 of them: 127, 183 and, with the 24-plane chunks chosen, 116 us.
+// Phase-field planes with interface nodes are several times slower, which
+// this does not see: 16 planes at most there.
+void ens_plan(tslb_ensemble* e) {
+    static const int cands[] = {8, 12, 16, 24, 32, 48, 64, 1 << 20};
+    double least = 1e300;
+    for (int zc : cands) {
+        if (e->mode == TSLB_MODE_PHASEFIELD && zc > 16) break;
+        std::map<int, long long, std::greater<int>> items;   // how many of each length, longest first
+        for (const tslb_ctx* c : e->m) {
+            const bool one = c->p.bc[0] == TSLB_BC_PERIODIC && c->nx <= 32;
+            const long long tx = one ? 1 : (c->nx + LXV - 1) / LXV;
+            const int th = even_rows(c->ny, SMALLW - 2), z = even_rows(c->nz, zc);
+            const long long cols = tx * ((c->ny + th - 1) / th);
+            items[z] += cols * (c->nz / z);
+            if (c->nz % z) items[c->nz % z] += cols;
+        }
+        std::priority_queue<double, std::vector<double>, std::greater<double>> busy;   // blocks by when they are free
+        for (int b = 0; b < e->grid; ++b) busy.push(0.0);
+        double rounds = 0.0, rest = 0.0;
+        for (const auto& it : items) {
+            const double t = it.first + 3.0;
+            rounds += (double)(it.second / e->grid) * t;   // every block one item of this length
+            for (long long k = it.second % e->grid; k > 0; --k) {
+                const double end = busy.top() + t;
+                busy.pop();
+                busy.push(end);
+                rest = std::max(rest, end);
+            }
+        }
+        if (rounds + rest < least) {
+            least = rounds + rest;
+            e->zchunk = zc;
+        }
+    }
 }
 
 // The ensemble kernel of the ensemble's mode, storage and x alignment:
@@ -1880,6 +1926,7 @@ int tslb_ensemble_create(const tslb_params* params, const int* dims, int n, tslb
         return efail(nullptr, TSLB_ERR_CUDA, msg);
     }
     e->grid = kEnsBlocksPerSM * e->sms;  // persistent: the resident blocks walk the work list
+    ens_plan(e);
     int rc = ens_build(e);
     if (rc) {
         std::string msg = e->err;
