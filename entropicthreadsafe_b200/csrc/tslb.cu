@@ -691,8 +691,9 @@ int launch_normals(tslb_ctx* c) {
 // correction and solid mask of `a`.  launch = false only sets its shared
 // memory attribute.  Returns the error of that attribute; launch errors are
 // left to cudaGetLastError.
-cudaError_t launch_step_kernel(const StepArgs& a, int mode, int prec, cudaStream_t st, bool launch = true) {
-    return tslb_launch::scalar_step(a, mode, prec, st, launch);
+cudaError_t launch_step_kernel(const StepArgs& a, int mode, int prec, cudaStream_t st, bool launch = true,
+                               bool early = false) {
+    return tslb_launch::scalar_step(a, mode, prec, st, launch, early);
 }
 
 int launch_moment_bcs(tslb_ctx* c) {
@@ -723,7 +724,8 @@ int launch_step(tslb_ctx* c) {
         if (rc) return rc;
     }
     StepArgs a = make_args(c, c->state[c->cur], c->state[c->cur ^ 1]);
-    CUDA_TRY(c, launch_step_kernel(a, c->p.mode, c->p.precision, c->stream));
+    // (a slab's step follows the halo exchange in plain order)
+    CUDA_TRY(c, launch_step_kernel(a, c->p.mode, c->p.precision, c->stream, true, c->halo == 0));
     c->launches++;
     CUDA_TRY(c, cudaGetLastError());
     c->cur ^= 1;
@@ -1545,7 +1547,7 @@ extern "C" int tslb_step_noalloc(const tslb_params* p, int nx, int ny, int nz, c
     const StepPlan plan = step_plan(nx, ny, nz, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
     view.warps = plan.warps; view.th = plan.th; view.zchunk = plan.zchunk; view.grid = plan.grid;
     StepArgs a = make_args(&view, d_in, d_out);
-    if ((e = launch_step_kernel(a, p->mode, TSLB_PREC_FP32, st)) != cudaSuccess)
+    if ((e = launch_step_kernel(a, p->mode, TSLB_PREC_FP32, st, true, true)) != cudaSuccess)
         return noalloc_fail(TSLB_ERR_CUDA, std::string("step kernel attribute: ") + cudaGetErrorString(e));
     if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_fail(TSLB_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
     return TSLB_OK;

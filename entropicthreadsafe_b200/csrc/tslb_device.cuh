@@ -254,7 +254,7 @@ __device__ __forceinline__ float store_pair16(const StepArgs& a, unsigned int id
 
 template <class T>
 __device__ __forceinline__ float ld_field(const StepArgs& a, int f, long long idx) {
-    return cvt_in<T>(__ldg(reinterpret_cast<const T*>(a.in) + f * a.N + idx), a, f);
+    return cvt_in<T>(reinterpret_cast<const T*>(a.in)[f * a.N + idx], a, f);
 }
 
 template <class T>

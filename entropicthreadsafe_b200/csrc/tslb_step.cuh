@@ -720,9 +720,9 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
                 if (e.x >= 0) cp_async4(slot + e.x, phin + (zoff + e.y));
             }
         } else {
-            p.own = cvt_in<T>(__ldg(phin + (zoff + n0.off)), a, F_PHI);
+            p.own = cvt_in<T>(phin[zoff + n0.off], a, F_PHI);
 #pragma unroll
-            for (int k = 0; k < NEX; ++k) p.ex[k] = cvt_in<T>(__ldg(phin + (zoff + exts[k * NT + tid].y)), a, F_PHI);
+            for (int k = 0; k < NEX; ++k) p.ex[k] = cvt_in<T>(phin[zoff + exts[k * NT + tid].y], a, F_PHI);
         }
     };
     // A warp's chunk reads of a plane: lanes below 30 read chunk lane % CPR of
@@ -791,9 +791,9 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
                     if (e.x >= 0) cp_async4(slot + e.x, phin + (zoff + e.y));
                 }
             } else {
-                p.own = cvt_in<T>(__ldg(phin + (zoff + n0.off)), a, F_PHI);
+                p.own = cvt_in<T>(phin[zoff + n0.off], a, F_PHI);
 #pragma unroll
-                for (int k = 0; k < NEX; ++k) p.ex[k] = cvt_in<T>(__ldg(phin + (zoff + exts[k * NT + tid].y)), a, F_PHI);
+                for (int k = 0; k < NEX; ++k) p.ex[k] = cvt_in<T>(phin[zoff + exts[k * NT + tid].y], a, F_PHI);
             }
         } else if (PHI) {
             if (pchunks && !slow && (a.phi_mirror || !zbehind(zp))) {
@@ -855,6 +855,10 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         cslot = atomicAdd(&cq_n[z & 1], 1);
         cq_list[(z & 1) * NT + cslot] = (unsigned short)tid;
     };
+
+    // The step may have been launched while the kernel before it still runs: the
+    // indices above are its own, all that follows reads what that kernel wrote.
+    cudaGridDependencySynchronize();
 
     // prologue: the phi planes the first source plane reads, its moments
     for (int z = z0 - 1 - RIM; z <= z0 - 1 + RIM; ++z) {
@@ -1214,6 +1218,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
 // in one piece or, across the end of a tile, in several.
 template <int MODE, class T, int W, bool TAU = false, bool SOLID = false>
 __global__ void __launch_bounds__(32 * W, BIGW / W) step_kernel(const __grid_constant__ StepArgs a) {
+    cudaTriggerProgrammaticLaunchCompletion();   // the next step may start; it waits as this one does
     const int planes = a.zt1 - a.zt0, tx = a.xwrap ? 1 : (a.nx + LXV - 1) / LXV, ty = (a.ny + a.th - 1) / a.th;
     const int bx = blockIdx.x % tx, b = blockIdx.x / tx;
     int p, end;   // the block's part of the sequence
