@@ -17,27 +17,11 @@ cudaError_t scalar_step(const tslb::StepArgs& a, int mode, int prec, cudaStream_
     using namespace tslb;
     const unsigned grid = a.zchunk > 0 ? (unsigned)(tiles_x(a) * tiles_y(a) * ((a.zt1 - a.zt0 + a.zchunk - 1) / a.zchunk)) : (unsigned)a.grid;
     cudaError_t err = cudaSuccess;
-    if (launch && early) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();   // the launch reports it
-        else early = cap == cudaStreamCaptureStatusNone;
-    }
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
     auto with_warps = [&](auto warps) {
         constexpr int W = decltype(warps)::value;
         auto go = [&](void (*kernel)(const StepArgs), int sm) {
             err = ensure_smem_attr((const void*)kernel, sm);
-            if (err != cudaSuccess || !launch) return;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(grid);
-            cfg.blockDim = dim3(32, W, 1);
-            cfg.dynamicSmemBytes = sm;
-            cfg.stream = st;
-            cfg.attrs = &at;
-            cfg.numAttrs = early ? 1 : 0;
-            cudaLaunchKernelEx(&cfg, kernel, a);   // its error is left to cudaGetLastError
+            if (err == cudaSuccess && launch) launch_after(kernel, grid, dim3(32, W, 1), sm, st, early, a);
         };
         constexpr int C = TSLB_MODE_COLOUR, P = TSLB_MODE_PHASEFIELD, S = TSLB_MODE_SINGLE;
         with_storage(prec, [&](auto tag) {

@@ -261,11 +261,13 @@ __global__ void pops_to_moments_kernel(int nx, int ny, int nz, long long N, int 
 constexpr int RED_SLOTS = 12, RED_PARTS = RED_SLOTS + 1, RED_THREADS = 256;
 struct RedScale { float d, u, v, w, phi; };
 template <class T>
-__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(const T* __restrict__ s, long long n, long long N,
+__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(const T* s, long long n, long long N,
                                                              RedScale sc, int colour, double* part, double* out,
                                                              unsigned int* ticket) {
     __shared__ double sh[RED_PARTS][RED_THREADS / 32];
     __shared__ bool last;
+    cudaTriggerProgrammaticLaunchCompletion();   // the next step may start; it waits for this kernel
+    cudaGridDependencySynchronize();             // (and this one for the step before)
     double acc[RED_SLOTS];
     for (int k = 0; k < RED_SLOTS; ++k) acc[k] = 0.0;
     float umax2 = 0.f;
@@ -1092,8 +1094,9 @@ int enqueue_reduce(tslb_ctx* c, double* host_dst) {
     const RedScale sc{1.0f / c->scale[F_D], 1.0f / c->scale[F_U], 1.0f / c->scale[F_V], 1.0f / c->scale[F_W], 1.0f / c->scale[F_PHI]};
     with_storage(c->p.precision, [&](auto tag) {
         using T = decltype(tag);
-        reduce_kernel<T><<<blocks, RED_THREADS, 0, c->stream>>>(static_cast<const T*>(c->state[c->cur]) + off, n, c->N, sc,
-                                                                c->p.mode == TSLB_MODE_COLOUR, c->red, host_dst, ticket);
+        tslb_launch::launch_after(reduce_kernel<T>, blocks, dim3(RED_THREADS), 0, c->stream, c->halo == 0,
+                                  static_cast<const T*>(c->state[c->cur]) + off, n, c->N, sc,
+                                  c->p.mode == TSLB_MODE_COLOUR, c->red, host_dst, ticket);
     });
     c->launches++;
     CUDA_TRY(c, cudaGetLastError());
