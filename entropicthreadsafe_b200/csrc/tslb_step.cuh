@@ -35,7 +35,7 @@
 // exist in memory.
 //
 // What bounds it: the latency of the chain through a plane, not HBM.  On the
-// 384 x 192 x 128 colour channel (FP32) a step takes 0.35 ms on a B200, where
+// 384 x 192 x 128 colour channel (FP32) a step takes 0.33 ms on a B200, where
 // the kernel that pulled 27 populations took 0.45 ms (1109 thread instructions
 // a node, issue active 62%) and 88 B a node at the measured copy rate take
 // 0.129 ms.  A warp spends 572 instructions on a row and plane (640 a target
