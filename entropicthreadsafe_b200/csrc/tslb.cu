@@ -634,16 +634,16 @@ int even_rows(int ny, int most) {   // tiles of equal height, at most `most` row
     return (ny + tiles - 1) / tiles;
 }
 
-// The plan with the least estimated time, in microseconds on a B200.  A block
+// The plan with the least estimated time, about microseconds on a B200.  A block
 // takes `plane` per source plane and about `extra` planes' time outside its
 // target planes (two more source planes, its start); blocks run in waves.
 // Measured on the 384 x 192 x 128 colour channel: 16-warp blocks in 32 / 16 / 8
-// plane chunks 0.350 / 0.379 / 0.442 ms, which is 2.0 us a plane and 3 planes
-// extra; two 8-warp blocks on an SM 1.72 us a plane, of fewer rows (6 of 8 are
+// plane chunks 0.333 / 0.355 / 0.404 ms, 8-warp blocks in 64 / 32 / 16 plane
+// chunks 0.331 / 0.340 / 0.352 ms: 3 planes extra, and a plane of two 8-warp
+// blocks on an SM takes 0.85 of one of 16 warps, with fewer rows (6 of 8 are
 // targets, against 14 of 16).  Equal shares have no last wave, but their blocks
 // are at different planes and share less of what they read: 8% slower a plane
-// (0.373 ms on the channel, where chunks fill 4.92 waves; 52 against 58 us on a
-// 173 x 59 x 91 Couette cell).  The phase field takes chunks only, and short
+// (48 against 51 us in the best chunks on a 173 x 59 x 91 Couette cell).  The phase field takes chunks only, and short
 // ones: planes with interface nodes are about three times slower, so the last
 // blocks to finish are those across a droplet, by their length (96^3 with one
 // droplet: 130 us in 24-plane chunks).
