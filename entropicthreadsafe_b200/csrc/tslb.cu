@@ -289,9 +289,45 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(const T* s, long lo
         else return Stor<T>::ld(x);
     };
     // several nodes' loads in flight per thread, then their FP64 accumulation
-    constexpr int U4 = sizeof(T) == 4 ? 4 : 8;
+    constexpr int U4 = 4;
     const long long S = (long long)gridDim.x * blockDim.x;
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if constexpr (sizeof(T) == 2) {
+        // 16-bit nodes two a load where the fields start on whole words (not so
+        // for a slab of odd planes): 42.8 us on the 384 x 192 x 128 channel, FP32 41.8,
+        // one by one 62.7
+        if (!(reinterpret_cast<uintptr_t>(s) & 3) && !(N & 1)) {
+            auto load = [&](long long j, unsigned x[5]) {
+                x[0] = __ldcs(reinterpret_cast<const unsigned*>(s + F_D * N) + j);
+                x[1] = __ldcs(reinterpret_cast<const unsigned*>(s + F_U * N) + j);
+                x[2] = __ldcs(reinterpret_cast<const unsigned*>(s + F_V * N) + j);
+                x[3] = __ldcs(reinterpret_cast<const unsigned*>(s + F_W * N) + j);
+                x[4] = __ldcs(reinterpret_cast<const unsigned*>(s + F_PHI * N) + j);
+            };
+            auto both = [&](const unsigned x[5]) {
+#pragma unroll
+                for (int h = 0; h < 32; h += 16) {
+                    auto at = [&](int f, float scale) { return val(bits_as<T>((unsigned short)(x[f] >> h)), scale); };
+                    node(at(0, sc.d), at(1, sc.u), at(2, sc.v), at(3, sc.w), at(4, sc.phi));
+                }
+            };
+            const long long n2 = n / 2;
+            for (; i + (U4 - 1) * S < n2; i += U4 * S) {
+                unsigned x[U4][5];
+#pragma unroll
+                for (int q = 0; q < U4; ++q) load(i + q * S, x[q]);
+#pragma unroll
+                for (int q = 0; q < U4; ++q) both(x[q]);
+            }
+            for (; i < n2; i += S) {
+                unsigned x[5];
+                load(i, x);
+                both(x);
+            }
+            // an odd last node, by the thread whose next pair it would begin
+            i = i == n2 && (n & 1) ? n - 1 : n;
+        }
+    }
     for (; i + (U4 - 1) * S < n; i += U4 * S) {
         T x[U4][5];
 #pragma unroll
