@@ -660,12 +660,14 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     const int X0 = X - lane;
     const int Xm = X0 & ~(EPC - 1), Xp = (X0 - RIM) & ~3;        // first columns read (moments, phi)
     const bool chunks = !a.xwrap && a.nx % EPC == 0 && X0 - RIM >= 0 && max(Xm, Xp) + ROWE <= a.nx;
-    const bool pchunks = PHI && ASYNC && chunks;
+    const bool yin = yper || (y0 - 1 - RIM >= 0 && y0 - 1 + W + RIM <= a.ny);   // no row behind a y face
+    // (a tile with computed ghost rows reads phi node by node in every warp: a rim
+    // node belongs to another warp than the row it ends, so a block reads in one way)
+    const bool pchunks = PHI && ASYNC && chunks && (a.phi_mirror || yin);
     // inner: no node of the tile or its rim lies behind a face; then the planes
     // whose neighbours and reads ahead are planes of the lattice as they stand
     // take the iteration without those cases
-    const bool inner = !SOLID && !a.xwrap && (xper || (X0 - RIM >= 0 && X0 + 32 + RIM <= a.nx)) &&
-                       (yper || (y0 - 1 - RIM >= 0 && y0 - 1 + W + RIM <= a.ny));
+    const bool inner = !SOLID && !a.xwrap && (xper || (X0 - RIM >= 0 && X0 + 32 + RIM <= a.nx)) && yin;
 
     // ---- phi ring: this thread fills its own node and up to NEX rim nodes ----
     const int rx = pchunks ? X0 - RIM - Xp : 0;   // ring column of the tile's first phi column
@@ -810,7 +812,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
                 for (int k = 0; k < NEX; ++k) p.ex[k] = phi_raw(zoff + exts[k * NT + tid].y);
             }
         } else if (PHI) {
-            if (pchunks && !slow && (a.phi_mirror || !zbehind(zp))) {
+            if (pchunks && (a.phi_mirror || !zbehind(zp))) {   // (no ghost columns or rows: never `slow`)
                 const T* cpp = srcs[NT];
                 if (cpp) cp_async16(ring + cpr + (zp & (RING - 1)) * RAREA, cpp + (unsigned)zclamp(zp) * plane);
             } else {
