@@ -665,9 +665,10 @@ int ensure_normals(tslb_ctx* c) {
 struct StepPlan { int warps, th, zchunk, grid; };
 constexpr int kEnsBlocksPerSM = BIGW / SMALLW;   // ensemble blocks (SMALLW warps) resident on an SM
 
-int even_rows(int ny, int most) {   // tiles of equal height, at most `most` rows
-    const int tiles = (ny + most - 1) / most;
-    return (ny + tiles - 1) / tiles;
+int even_rows(int ny, int most) {   // tiles of equal height, at most `most` rows (any positive number)
+    most = std::min(most, ny);
+    const int tiles = (int)(((long long)ny + most - 1) / most);
+    return (int)(((long long)ny + tiles - 1) / tiles);
 }
 
 // The plan with the least estimated time, about microseconds on a B200.  A block
