@@ -229,10 +229,17 @@ __device__ __forceinline__ unsigned int sr_field(unsigned int hnode, int f) {
     unsigned int h = (hnode + (unsigned int)f * 0x9E3779B9u) * 0x85EBCA6Bu;
     return h ^ (h >> 16);
 }
+// the larger of two numbers, NaN if either is one (fmaxf drops a NaN)
+__device__ __forceinline__ float max_nan(float x, float y) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+}
 // Store fields f and g (g == f: f alone) of node id in 16-bit storage with
 // one paired conversion: cvt.rn / cvt.rs (stochastic, random bits r) to
 // f16x2 or bf16x2 of the stored values (fp16: value * per-field scale).
-// Returns the largest stored magnitude before rounding, for the range check.
+// Returns the largest stored magnitude before rounding (NaN if either is), for
+// the range check.
 template <class T>
 __device__ __forceinline__ float store_pair16(const StepArgs& a, unsigned int id, int f, int g, float vf, float vg, int sr,
                                               unsigned int r) {
@@ -249,7 +256,7 @@ __device__ __forceinline__ float store_pair16(const StepArgs& a, unsigned int id
     // the low half holds field f, the high half field g
     static_cast<T*>(a.fo[f])[id] = bits_as<T>((unsigned short)(d & 0xFFFFu));
     if (g != f) static_cast<T*>(a.fo[g])[id] = bits_as<T>((unsigned short)(d >> 16));
-    return fmaxf(fabsf(xf), fabsf(xg));
+    return max_nan(fabsf(xf), fabsf(xg));
 }
 
 template <class T>

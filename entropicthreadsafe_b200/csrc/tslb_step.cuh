@@ -569,7 +569,7 @@ __device__ __forceinline__ void store_target(const StepArgs& a, unsigned int id,
 #pragma unroll
         for (int f = 0; f < nout; f += 2) {
             const int g = f + 1 < nout ? f + 1 : f;
-            vmax = fmaxf(vmax, store_pair16<T>(a, id, f, g, o[f], o[g], a.sr, sr_field(hnode, f)));
+            vmax = max_nan(vmax, store_pair16<T>(a, id, f, g, o[f], o[g], a.sr, sr_field(hnode, f)));
         }
         // non-finite, or beyond the storage's range (NaN fails the comparison)
         bad = !(vmax <= Stor16Max<T>::value);
