@@ -1,6 +1,6 @@
 // step_launch.h -- host-side launchers of the step and ensemble kernels,
-// whose instantiations live in a translation unit of their own (k_scalar.cu)
-// that compiles in parallel with the rest.  Every launcher with launch =
+// whose instantiations live in translation units of their own (k_scalar.cu,
+// k_inlet.cu, k_general.cu) that compile in parallel with the rest.  Every launcher with launch =
 // false only sets the kernel's shared-memory attribute (before a stream
 // capture, for instance).
 #pragma once
@@ -47,7 +47,8 @@ void launch_after(void (*kernel)(P...), unsigned grid, dim3 block, size_t smem, 
 // step kernel (tslb_step.cuh): every storage type, tau correction and
 // interior solid mask (early: see launch_after)
 cudaError_t scalar_step(const tslb::StepArgs& a, int mode, int prec, cudaStream_t st, bool launch, bool early = false);
-cudaError_t scalar_ensemble(const tslb::StepArgs* args, const tslb::WorkItem* work, int nwork, int grid, int mode,
-                            int prec, unsigned int* step, cudaStream_t st, bool launch);
+// general: the largest StepArgs::general of the members
+cudaError_t scalar_ensemble(const tslb::StepArgs* args, const tslb::WorkItem* work, int nwork, int grid, int mode, int prec,
+                            int general, unsigned int* step, cudaStream_t st, bool launch);
 
 }  // namespace tslb_launch

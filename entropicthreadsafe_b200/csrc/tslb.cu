@@ -84,6 +84,27 @@ int validate(const tslb_params* p, int nx, int ny, int nz, std::string& why) {
     return TSLB_OK;
 }
 
+// Which nodes of a lattice have no closed sums of the populations from behind their
+// faces (StepArgs::general): 1 those at one inlet or outlet face normal to y or z;
+// 2 also those at inlets and outlets normal to x, at edges that are not all
+// bounce-back, between two faces of one axis, and at faces with interior solids that
+// are not bounce-back.
+int general_nodes(const tslb_params& p, int nx, int ny, int nz, bool solids) {
+    int axes = 0;
+    bool io = false, xio = false, bounce = true, thin = false;
+    for (int f = 0; f < 6; ++f) {
+        const int k = p.bc[f];
+        if (k == TSLB_BC_PERIODIC) continue;
+        axes += f & 1;
+        const bool through = k == TSLB_BC_INLET || k == TSLB_BC_OUTLET;
+        io = io || through;
+        xio = xio || (through && f < 2);
+        bounce = bounce && k == TSLB_BC_BOUNCEBACK;
+        thin = thin || (f < 2 ? nx : f < 4 ? ny : nz) == 1;
+    }
+    return xio || thin || (!bounce && (axes > 1 || (axes > 0 && solids))) ? 2 : io ? 1 : 0;
+}
+
 StepArgs make_args(tslb_ctx* c, const void* in, void* out) {
     StepArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -123,6 +144,7 @@ StepArgs make_args(tslb_ctx* c, const void* in, void* out) {
     a.dtau = c->closure ? c->dtau : (c->base_on ? c->dtau_base : nullptr);
     a.solid = c->solid_on ? c->solid : nullptr;
     a.near = c->solid_on ? c->near : nullptr;
+    a.general = general_nodes(c->p, c->nx, c->ny, c->nz, c->solid_on);
     a.sr = 1;
     a.sr_step = (unsigned int)c->steps_done;
     a.sr_counter = nullptr;
@@ -671,6 +693,11 @@ int even_rows(int ny, int most) {   // tiles of equal height, at most `most` row
     return (int)(((long long)ny + tiles - 1) / tiles);
 }
 
+// some tiles' boundary nodes make all their planes slower than other tiles'
+bool slow_columns(const tslb_params& p, int nx, int ny, int nz, bool solids) {
+    return general_nodes(p, nx, ny, nz, solids) && (p.bc[0] != TSLB_BC_PERIODIC || p.bc[2] != TSLB_BC_PERIODIC);
+}
+
 // The plan with the least estimated time, about microseconds on a B200.  A block
 // takes `plane` per source plane and about `extra` planes' time outside its
 // target planes (two more source planes, its start); blocks run in waves.
@@ -683,10 +710,12 @@ int even_rows(int ny, int most) {   // tiles of equal height, at most `most` row
 // (48 against 51 us in the best chunks on a 173 x 59 x 91 Couette cell).  The phase field takes chunks only, and short
 // ones: planes with interface nodes are about three times slower, so the last
 // blocks to finish are those across a droplet, by their length (96^3 with one
-// droplet: 130 us in 24-plane chunks).
-StepPlan step_plan(int nx, int ny, int nz, bool xper, int sms, int mode) {
+// droplet: 130 us in 24-plane chunks).  So do lattices with interior solids or with
+// nodes on the general boundary path at x or y faces, whose tiles are the slow ones.
+StepPlan step_plan(int nx, int ny, int nz, const tslb_params& p, bool solids, int sms) {
     StepPlan best{BIGW, 1, nz, 0};
     double least = 1e300;
+    const bool xper = p.bc[0] == TSLB_BC_PERIODIC, uneven = p.mode == TSLB_MODE_PHASEFIELD || solids || slow_columns(p, nx, ny, nz, solids);
     const long long tx = (xper && nx <= 32) ? 1 : (nx + LXV - 1) / LXV;
     constexpr double extra = 3.0;
     for (int w : {BIGW, SMALLW}) {
@@ -696,19 +725,27 @@ StepPlan step_plan(int nx, int ny, int nz, bool xper, int sms, int mode) {
         for (int nc = 1; nc <= nz; ++nc) {
             const int zc = (nz + nc - 1) / nc;
             const long long blocks = tx * ty * ((nz + zc - 1) / zc);
-            const double tail = mode == TSLB_MODE_PHASEFIELD ? 3.0 * zc : 0.0;
+            const double tail = uneven ? 3.0 * zc : 0.0;
             const double cost = (double)((blocks + slots - 1) / slots) * (zc + extra) * plane(blocks) + tail;
             if (cost < least) { least = cost; best = StepPlan{w, th, zc, 0}; }
             if (nc > 1 && blocks > 16 * slots) break;   // more waves only add planes outside the chunks
         }
         const long long parts = std::min(slots / tx, ty * nz);
-        if (mode != TSLB_MODE_PHASEFIELD && parts > 0 && ty * nz < (1LL << 31)) {
+        if (!uneven && parts > 0 && ty * nz < (1LL << 31)) {
             const double share = (double)(ty * nz) / parts;
             const double cost = 1.08 * (share + extra * (share / nz + 1.0)) * plane(parts * tx);
             if (cost < least) { least = cost; best = StepPlan{w, th, 0, (int)(parts * tx)}; }
         }
     }
     return best;
+}
+
+// The plan of a context's step, for the planes it updates and its solid nodes.
+void plan_step(tslb_ctx* c) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const StepPlan plan = step_plan(c->nx, c->ny, (c->zt1 > 0 ? c->zt1 : c->nz) - c->zt0, c->p, c->solid_on, sms);
+    c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
 }
 
 int launch_normals(tslb_ctx* c) {
@@ -931,10 +968,7 @@ int tslb_create(const tslb_params* p, int nx, int ny, int nz, tslb_ctx** out) {
     }
     // the pool's allocations and the clears are ordered on the lattice's stream: complete them for every stream
     if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return bail(e, "cudaStreamSynchronize");
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const StepPlan plan = step_plan(nx, ny, nz, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
-    c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
+    plan_step(c);
     if ((e = launch_step_kernel(make_args(c, c->state[0], c->state[1]), p->mode, p->precision, c->stream, false)) != cudaSuccess)
         return bail(e, "cudaFuncSetAttribute");
     *out = c;
@@ -1246,6 +1280,7 @@ int tslb_set_solid_mask(tslb_ctx* c, const unsigned char* isfluid) {
     if (!c) return TSLB_ERR_ARG;
     if (!isfluid) {
         c->solid_on = false;
+        plan_step(c);
         return TSLB_OK;
     }
     if (c->p.precision != TSLB_PREC_FP32)
@@ -1270,6 +1305,7 @@ int tslb_set_solid_mask(tslb_ctx* c, const unsigned char* isfluid) {
     cudaFree(d);
     if (e != cudaSuccess) return fail(c, TSLB_ERR_CUDA, std::string("tslb_set_solid_mask: ") + cudaGetErrorString(e));
     c->solid_on = true;
+    plan_step(c);
     return tslb_internal::prepare_step_kernel(c);
 }
 
@@ -1526,10 +1562,12 @@ int noalloc_setup(int dev, NoallocScratch** out) {
             StepArgs a;
             std::memset(&a, 0, sizeof(a));
             a.nx = a.ny = a.nz = a.zchunk = a.th = 1;
-            for (int w : {BIGW, SMALLW}) {
-                a.warps = w;
-                if (e == cudaSuccess) e = launch_step_kernel(a, mode, TSLB_PREC_FP32, nullptr, false);
-            }
+            for (int w : {BIGW, SMALLW})
+                for (int general : {0, 1, 2}) {
+                    a.warps = w;
+                    a.general = general;
+                    if (e == cudaSuccess) e = launch_step_kernel(a, mode, TSLB_PREC_FP32, nullptr, false);
+                }
             if (e != cudaSuccess) return noalloc_fail(TSLB_ERR_CUDA, std::string("step kernel attribute: ") + cudaGetErrorString(e));
         }
         s.ready = true;
@@ -1584,7 +1622,7 @@ extern "C" int tslb_step_noalloc(const tslb_params* p, int nx, int ny, int nz, c
     for (int f = 0; f < NF; ++f) view.scale[f] = 1.0f;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const StepPlan plan = step_plan(nx, ny, nz, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
+    const StepPlan plan = step_plan(nx, ny, nz, *p, false, sms);
     view.warps = plan.warps; view.th = plan.th; view.zchunk = plan.zchunk; view.grid = plan.grid;
     StepArgs a = make_args(&view, d_in, d_out);
     if ((e = launch_step_kernel(a, p->mode, TSLB_PREC_FP32, st, true, true)) != cudaSuccess)
@@ -1729,10 +1767,7 @@ int tslb_create_slab(const tslb_params* p, int nx, int ny, int nz, int z_begin, 
     c->halo_hi = hi;
     c->zt0 = lo;
     c->zt1 = lo + (z_end - z_begin);
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const StepPlan plan = step_plan(nx, ny, z_end - z_begin, p->bc[0] == TSLB_BC_PERIODIC, sms, p->mode);
-    c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
+    plan_step(c);
     *out = c;
     return TSLB_OK;
 }
@@ -1768,6 +1803,7 @@ struct tslb_ensemble {
     StepArgs* d_args[2] = {nullptr, nullptr};  // per step parity: member args
     WorkItem* d_work = nullptr;
     int nwork = 0;
+    int general = 0;                   // the largest StepArgs::general of the members
     int zchunk = 16;                   // most target planes of an item
     int grid = 0;                      // 0: one block per work item
     int sms = 148;
@@ -1895,7 +1931,7 @@ void ens_plan(tslb_ensemble* e) {
 cudaError_t ens_kernel(tslb_ensemble* e, bool launch) {
     const int grid = e->grid > 0 ? std::min(e->grid, e->nwork) : e->nwork;
     const StepArgs* args = e->d_args[e->parity];
-    return tslb_launch::scalar_ensemble(args, e->d_work, e->nwork, grid, e->mode, e->precision, e->d_step,
+    return tslb_launch::scalar_ensemble(args, e->d_work, e->nwork, grid, e->mode, e->precision, e->general, e->d_step,
                                         e->stream, launch);
 }
 
@@ -1953,6 +1989,7 @@ int tslb_ensemble_create(const tslb_params* params, const int* dims, int n, tslb
             return efail(nullptr, rc, msg);
         }
         e->m.push_back(c);
+        e->general = std::max(e->general, general_nodes(c->p, c->nx, c->ny, c->nz, false));
     }
     cudaError_t ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
     // step counter of the stochastic rounding (members start at step 0) and launch ticket

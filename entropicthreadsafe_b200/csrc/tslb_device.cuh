@@ -77,6 +77,8 @@ struct StepArgs {
     int th;                 // target rows of a tile, at most warps - 2
     int xwrap;              // a warp holds the whole periodic x axis (nx <= 32)
     int phi_mirror;         // ghost phi is the nearest node's on every face that is not periodic
+    int general;            // nodes without closed boundary sums: 0 none, 1 at single inlet or outlet faces
+                            // normal to y or z (io_face), 2 others too (direction_from_behind)
     int mode;
     float omega_pf;         // 1/tau (phase field)
     float inv_nu_a, inv_nu_b;  // colour: 1/nu of each component
@@ -502,7 +504,7 @@ __device__ __forceinline__ float eval_P(const float* K, long long stride, int cx
 
 // accumulate population value f (already weighted) of direction c into acc
 template <class Acc>
-__device__ __forceinline__ void acc_dir_rt(const Acc& acc, int cx, int cy, int cz, float f) {
+__device__ __forceinline__ void acc_dir_rt(Acc&& acc, int cx, int cy, int cz, float f) {
     acc[A_RHO] += f;
     acc[A_JX] += cx * f; acc[A_JY] += cy * f; acc[A_JZ] += cz * f;
     acc[A_XX] += (cx * cx) * f; acc[A_YY] += (cy * cy) * f; acc[A_ZZ] += (cz * cz) * f;

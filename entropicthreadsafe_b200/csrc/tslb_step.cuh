@@ -194,161 +194,219 @@ __device__ __forceinline__ void face_target(const StepArgs& a, const float* K, c
     }
 }
 
-// Regularized or bounce-back populations entering target (x,y,z) from
-// behind non-periodic faces or from interior solids, direction by direction,
-// added to acc (in shared memory: registers are short where this runs); Kp holds
-// the target's own coefficients.  The general path, for edges of faces of
-// different kinds, inlets, outlets and interior solids; single walls and
-// bounce-back edges have closed sums above (a 173 x 59 x 91 Couette cell with
-// this path at its walls 70 us a step, with closed sums 52).
+// accumulators in shared memory, S apart (registers are short where they are used)
 template <int S>
 struct Strided {
     float* p;
     __device__ __forceinline__ float& operator[](int i) const { return p[i * S]; }
 };
-template <int MODE, class T, bool TAU, bool SOLID, class Acc>
-__device__ __forceinline__ void boundary_target(const StepArgs& a, const float* Kp, unsigned mask, int x, int y, int z,
-                                                const Acc& acc) {
+
+// The populations of one node from behind non-periodic faces or from interior
+// solids, the general path: edges of faces of different kinds, inlets, outlets,
+// and face nodes beside interior solids.  Single walls, bounce-back edges and
+// nodes beside solids only have closed or shorter sums of their own.
+// A node's 26 directions are a chain of about 26,000 cycles when one thread takes
+// them in turn, and its block waits at the plane barrier for it.  So the nodes are
+// listed, and the block's warps share them, half a warp a node and a lane a
+// direction (9 at a face, 15 at an edge, 19 at a corner): 160 x 128 x 96
+// colour steps with outlets normal to x / edges of bounce-back and moving walls took
+// 941 / 821 us in turn and take 195 / 179 us.
+// The directions, as bits of a 3 x 3 x 3 index, whose source lies behind one of the
+// faces of mask.
+__device__ __forceinline__ unsigned directions_behind(unsigned mask) {
+    constexpr unsigned xm = 0x1249249u, ym = 0x1c0e07u, zm = 0x1ffu;   // c = -1 along x, y, z
+    return (mask & 1u ? xm << 2 : 0u) | (mask & 2u ? xm : 0u) | (mask & 4u ? ym << 6 : 0u) | (mask & 8u ? ym : 0u) |
+           (mask & 16u ? zm << 18 : 0u) | (mask & 32u ? zm : 0u);
+}
+// position of set bit k (from 0) of b
+__device__ __forceinline__ int nth_bit(unsigned b, int k) {
+    int pos = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const int c = __popc(b >> pos & ((1u << w) - 1u));
+        if (k >= c) { k -= c; pos += w; }
+    }
+    return pos;
+}
+// Direction q of them (a 3 x 3 x 3 index): the population's value f and what it
+// adds to the colour sum.  Kp, stride: the node's coefficients; mom(f): its moments;
+// dt: its correction of the relaxation time.
+struct Incoming {
+    float f, col;
+};
+template <int MODE, class T, bool SOLID, class Mom>
+__device__ __forceinline__ Incoming direction_from_behind(const StepArgs& a, const float* Kp, int stride, unsigned mask, int x,
+                                                          int y, int z, int q, const Mom& mom, float dt) {
+    Incoming r{0.f, 0.f};
     // colour mode accumulates colour increments over the target's own phi
-    const float pht = Kp[K_C0];
-    // own raw moments (velocity faces only)
-    float m[NF];
-    bool have_m = false;
-    for (int q = 0; q < 27; ++q) {
-        // the 26 moving directions as a 3x3x3 index (q == 13 is the rest population)
-        const int dx = (q % 3) - 1, dy = ((q / 3) % 3) - 1, dz = (q / 9) - 1;
-        if (dx == 0 && dy == 0 && dz == 0) continue;
-        const int c[3] = {dx, dy, dz};
-        // face through which the source x - c lies: axis a, side (c>0 -> minus face)
-        int vface = -1;
-        bool solid = false;
+    const float pht = Kp[K_C0 * stride];
+    const int dx = (q % 3) - 1, dy = ((q / 3) % 3) - 1, dz = (q / 9) - 1;
+    const int c[3] = {dx, dy, dz};
+    // face through which the source x - c lies: axis a, side (c>0 -> minus face)
+    int vface = -1;
+    bool solid = false;
 #pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            if (c[ax] == 0) continue;
-            const int f = 2 * ax + (c[ax] > 0 ? 0 : 1);
-            if (mask & (1u << f)) {
-                solid = true;
-                const int k = a.face[f].kind;
-                // a later velocity face wins, as the oracle's face loop overwrites in face order
-                if (k == TSLB_BC_VELOCITY || k == TSLB_BC_INLET || k == TSLB_BC_OUTLET || k == TSLB_BC_PRESSURE) vface = f;
-            }
-        }
-        // an interior solid source node (the lattice's solid mask), periodic axes wrapped
-        bool msolid = false;
-        if (SOLID && !solid) {
-            const int sx = x - dx, sy = y - dy, sz = z - dz;
-            msolid = bit_at(a.solid, nidx(a, sx < 0 ? sx + a.nx : (sx >= a.nx ? sx - a.nx : sx),
-                                          sy < 0 ? sy + a.ny : (sy >= a.ny ? sy - a.ny : sy),
-                                          sz < 0 ? sz + a.nz : (sz >= a.nz ? sz - a.nz : sz)));
-        }
-        if (!solid && !msolid) continue;
-        const int c2 = dx * dx + dy * dy + dz * dz;
-        const float wq = wclass(c2);
-        // The pull skips whole solid z planes, but a source behind an x or y
-        // face, or an interior solid node, is a zero-coefficient node it visited.
-        const bool xy_solid = (dx && (mask & (1u << (dx > 0 ? 0 : 1)))) || (dy && (mask & (1u << (dy > 0 ? 2 : 3))));
-        const bool zplane_solid = a.face[4].kind != TSLB_BC_PERIODIC && (z - dz < 0 || z - dz >= a.nz);
-        const bool visited = (xy_solid && !zplane_solid) || msolid;
-        // colour mode: the visited zero node added w (0 - phi_t): undo it
-        if (MODE == TSLB_MODE_COLOUR && visited) acc[A_COL] += wq * pht;
-        if (vface < 0) {
-            // half-way bounce-back: f_c(x) = f^post_{-c}(x)
-            const float P = eval_P(Kp, 1, -dx, -dy, -dz);
-            acc_dir_rt(acc, dx, dy, dz, wq * P);
-            if (MODE == TSLB_MODE_COLOUR) {
-                // the reflected population carries the target's own colour: only the recolouring term
-                const float bc = -(dx * Kp[K_C1] + dy * Kp[K_C2] + dz * Kp[K_C3]);
-                acc[A_COL] += wq * invlen(c2) * bc;
-            } else if (MODE == TSLB_MODE_PHASEFIELD && c2 == 1) {
-                const float ge = -(dx * Kp[K_C1] + dy * Kp[K_C2] + dz * Kp[K_C3]);
-                acc[A_COL] += Kp[K_C0] + ge;
-            }
-        } else {
-            if (!have_m) {
-                const long long id = nidx(a, x, y, z);
-#pragma unroll
-                for (int f = 0; f < NF; ++f) m[f] = ld_field<T>(a, f, id);
-                have_m = true;
-            }
-            const FaceBC& fb = a.face[vface];
-            const int ax = vface >> 1;
-            float Ub[3] = {fb.u[0], fb.u[1], fb.u[2]};
-            float phib = fb.phi < -2.f ? m[F_PHI] : fb.phi;
-            // in-plane position of the ghost node the population leaves, x - c
-            // (periodic axes wrap, a non-periodic axis clamps), in the target's layer
-            int g[3] = {x, y, z};
-            {
-                const int cc[3] = {dx, dy, dz};
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    if (b == ax) continue;
-                    const int n = dimn(a, b), v = g[b] - cc[b];
-                    g[b] = (v >= 0 && v < n) ? v : (a.face[2 * b].kind == TSLB_BC_PERIODIC ? wrapi(v, n) : (v < 0 ? 0 : n - 1));
-                }
-            }
-            if (fb.kind == TSLB_BC_INLET) {
-                // the inlet plane at the ghost node (boundary_cds_3D_module.f90:934-986:
-                // u, v, w of node (i, j, 1) feed the populations it sends)
-                const long long pa = plane_area(a, vface), pi = plane_index(a, vface, g[0], g[1], g[2]);
-                Ub[0] = __ldg(fb.plane + pi);
-                Ub[1] = __ldg(fb.plane + pa + pi);
-                Ub[2] = __ldg(fb.plane + 2 * pa + pi);
-                phib = __ldg(fb.plane + 3 * pa + pi);
-            } else if (fb.kind == TSLB_BC_OUTLET || fb.kind == TSLB_BC_PRESSURE) {
-                phib = m[F_PHI];
-            }
-            float Uf[3] = {Ub[0], Ub[1], Ub[2]};  // velocity of the f equilibrium
-            if (fb.kind == TSLB_BC_OUTLET) {
-                // outlet: the normal velocity of the fluid node next to the ghost
-                // node (zero gradient, :992 w(i,j,nz) = w(i,j,nz-1))
-                Uf[ax] = ld_field<T>(a, F_U + ax, nidx(a, g[0], g[1], g[2]));
-            } else if (fb.kind == TSLB_BC_PRESSURE) {
-                // pressure outlet: the fluid node's velocity at density 1
-                Uf[0] = m[F_U]; Uf[1] = m[F_V]; Uf[2] = m[F_W];
-            }
-            const float d = fb.kind == TSLB_BC_PRESSURE ? 0.f : m[F_D], rho = 1.f + d;
-            float omega;
-            if (MODE == TSLB_MODE_COLOUR) {
-                const float ca = 0.5f * (1.f + m[F_PHI]), cb = 0.5f * (1.f - m[F_PHI]);
-                const float nu = 1.f / (ca * a.inv_nu_a + cb * a.inv_nu_b);
-                const float dt = TAU ? __ldg(a.dtau + nidx(a, x, y, z)) : 0.f;
-                omega = 2.f / (6.f * nu + 1.f + 2.f * dt);
-            } else {
-                omega = a.omega_pf;
-            }
-            // f^eq(rho, Ub)/w - 1 (boundary_cds_3D_module.f90:461-507)
-            const float cu = dx * Uf[0] + dy * Uf[1] + dz * Uf[2];
-            const float uu = Uf[0] * Uf[0] + Uf[1] * Uf[1] + Uf[2] * Uf[2];
-            const float t3 = 1.f / 3.f;
-            const float hxxy = (dx * dx - t3) * dy, hxxz = (dx * dx - t3) * dz, hxyy = (dy * dy - t3) * dx;
-            const float hyyz = (dy * dy - t3) * dz, hxzz = (dz * dz - t3) * dx, hyzz = (dz * dz - t3) * dy;
-            const float hxyz = (float)(dx * dy * dz);
-            const float U = Uf[0], V = Uf[1], W = Uf[2];
-            const float h3e = 13.5f * (hxxy * U * U * V + hxxz * U * U * W + hxyy * U * V * V + hyyz * V * V * W +
-                                       hxzz * U * W * W + hyzz * V * W * W) + 27.f * hxyz * U * V * W;
-            const float feqm1 = d + rho * (3.f * cu + 4.5f * cu * cu - 1.5f * uu + h3e);
-            // a^neq(Pi, u) of the fluid node
-            const float u = m[F_U], v = m[F_V], w = m[F_W];
-            const float pxx = m[F_XX], pxy = m[F_XY], pxz = m[F_XZ], pyy = m[F_YY], pyz = m[F_YZ], pzz = m[F_ZZ];
-            const float h2 = (dx * dx - t3) * pxx + (dy * dy - t3) * pyy + (dz * dz - t3) * pzz +
-                             2.f * (dx * dy * pxy + dx * dz * pxz + dy * dz * pyz);
-            const float an = 4.5f * h2 +
-                             13.5f * (hxxy * (2.f * u * pxy + v * pxx) + hxxz * (2.f * u * pxz + w * pxx) +
-                                      hxyy * (u * pyy + 2.f * v * pxy) + hyyz * (2.f * v * pyz + w * pyy) +
-                                      hxzz * (u * pzz + 2.f * w * pxz) + hyzz * (v * pzz + 2.f * w * pyz)) +
-                             27.f * hxyz * (u * pyz + v * pxz + w * pxy);
-            const float P = feqm1 + (1.f - omega) * an;
-            acc_dir_rt(acc, dx, dy, dz, wq * P);
-            if (MODE == TSLB_MODE_COLOUR) {
-                const float dphi = phib - pht;
-                acc[A_COL] += wq * fmaf(dphi, P, dphi);
-            } else if (MODE == TSLB_MODE_PHASEFIELD && c2 == 1) {
-                // g entering from the face (:984-986, :1044-1045)
-                const float eu = dx * Ub[0] + dy * Ub[1] + dz * Ub[2];
-                acc[A_COL] += 0.125f * phib * (1.f + 3.f * eu);
-            }
+    for (int ax = 0; ax < 3; ++ax) {
+        if (c[ax] == 0) continue;
+        const int f = 2 * ax + (c[ax] > 0 ? 0 : 1);
+        if (mask & (1u << f)) {
+            solid = true;
+            const int k = a.face[f].kind;
+            // a later velocity face wins, as the oracle's face loop overwrites in face order
+            if (k == TSLB_BC_VELOCITY || k == TSLB_BC_INLET || k == TSLB_BC_OUTLET || k == TSLB_BC_PRESSURE) vface = f;
         }
     }
+    // an interior solid source node (the lattice's solid mask), periodic axes wrapped
+    bool msolid = false;
+    if (SOLID && !solid) {
+        const int sx = x - dx, sy = y - dy, sz = z - dz;
+        msolid = bit_at(a.solid, nidx(a, sx < 0 ? sx + a.nx : (sx >= a.nx ? sx - a.nx : sx),
+                                      sy < 0 ? sy + a.ny : (sy >= a.ny ? sy - a.ny : sy),
+                                      sz < 0 ? sz + a.nz : (sz >= a.nz ? sz - a.nz : sz)));
+    }
+    if (!solid && !msolid) return r;
+    const int c2 = dx * dx + dy * dy + dz * dz;
+    const float wq = wclass(c2);
+    // The pull skips whole solid z planes, but a source behind an x or y
+    // face, or an interior solid node, is a zero-coefficient node it visited.
+    const bool xy_solid = (dx && (mask & (1u << (dx > 0 ? 0 : 1)))) || (dy && (mask & (1u << (dy > 0 ? 2 : 3))));
+    const bool zplane_solid = a.face[4].kind != TSLB_BC_PERIODIC && (z - dz < 0 || z - dz >= a.nz);
+    const bool visited = (xy_solid && !zplane_solid) || msolid;
+    // colour mode: the visited zero node added w (0 - phi_t): undo it
+    if (MODE == TSLB_MODE_COLOUR && visited) r.col += wq * pht;
+    if (vface < 0) {
+        // half-way bounce-back: f_c(x) = f^post_{-c}(x)
+        r.f = wq * eval_P(Kp, stride, -dx, -dy, -dz);
+        if (MODE == TSLB_MODE_COLOUR) {
+            // the reflected population carries the target's own colour: only the recolouring term
+            const float bc = -(dx * Kp[K_C1 * stride] + dy * Kp[K_C2 * stride] + dz * Kp[K_C3 * stride]);
+            r.col += wq * invlen(c2) * bc;
+        } else if (MODE == TSLB_MODE_PHASEFIELD && c2 == 1) {
+            const float ge = -(dx * Kp[K_C1 * stride] + dy * Kp[K_C2 * stride] + dz * Kp[K_C3 * stride]);
+            r.col += pht + ge;
+        }
+    } else {
+        float m[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) m[f] = mom(f);
+        const FaceBC& fb = a.face[vface];
+        const int ax = vface >> 1;
+        float Ub[3] = {fb.u[0], fb.u[1], fb.u[2]};
+        float phib = fb.phi < -2.f ? m[F_PHI] : fb.phi;
+        // in-plane position of the ghost node the population leaves, x - c
+        // (periodic axes wrap, a non-periodic axis clamps), in the target's layer
+        int g[3] = {x, y, z};
+        {
+            const int cc[3] = {dx, dy, dz};
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                if (b == ax) continue;
+                const int n = dimn(a, b), v = g[b] - cc[b];
+                g[b] = (v >= 0 && v < n) ? v : (a.face[2 * b].kind == TSLB_BC_PERIODIC ? wrapi(v, n) : (v < 0 ? 0 : n - 1));
+            }
+        }
+        if (fb.kind == TSLB_BC_INLET) {
+            // the inlet plane at the ghost node (boundary_cds_3D_module.f90:934-986:
+            // u, v, w of node (i, j, 1) feed the populations it sends)
+            const long long pa = plane_area(a, vface), pi = plane_index(a, vface, g[0], g[1], g[2]);
+            Ub[0] = __ldg(fb.plane + pi);
+            Ub[1] = __ldg(fb.plane + pa + pi);
+            Ub[2] = __ldg(fb.plane + 2 * pa + pi);
+            phib = __ldg(fb.plane + 3 * pa + pi);
+        } else if (fb.kind == TSLB_BC_OUTLET || fb.kind == TSLB_BC_PRESSURE) {
+            phib = m[F_PHI];
+        }
+        float Uf[3] = {Ub[0], Ub[1], Ub[2]};  // velocity of the f equilibrium
+        if (fb.kind == TSLB_BC_OUTLET) {
+            // outlet: the normal velocity of the fluid node next to the ghost
+            // node (zero gradient, :992 w(i,j,nz) = w(i,j,nz-1))
+            Uf[ax] = ld_field<T>(a, F_U + ax, nidx(a, g[0], g[1], g[2]));
+        } else if (fb.kind == TSLB_BC_PRESSURE) {
+            // pressure outlet: the fluid node's velocity at density 1
+            Uf[0] = m[F_U]; Uf[1] = m[F_V]; Uf[2] = m[F_W];
+        }
+        const float d = fb.kind == TSLB_BC_PRESSURE ? 0.f : m[F_D], rho = 1.f + d;
+        float omega;
+        if (MODE == TSLB_MODE_COLOUR) {
+            const float ca = 0.5f * (1.f + m[F_PHI]), cb = 0.5f * (1.f - m[F_PHI]);
+            const float nu = 1.f / (ca * a.inv_nu_a + cb * a.inv_nu_b);
+            omega = 2.f / (6.f * nu + 1.f + 2.f * dt);
+        } else {
+            omega = a.omega_pf;
+        }
+        // f^eq(rho, Ub)/w - 1 (boundary_cds_3D_module.f90:461-507)
+        const float cu = dx * Uf[0] + dy * Uf[1] + dz * Uf[2];
+        const float uu = Uf[0] * Uf[0] + Uf[1] * Uf[1] + Uf[2] * Uf[2];
+        const float t3 = 1.f / 3.f;
+        const float hxxy = (dx * dx - t3) * dy, hxxz = (dx * dx - t3) * dz, hxyy = (dy * dy - t3) * dx;
+        const float hyyz = (dy * dy - t3) * dz, hxzz = (dz * dz - t3) * dx, hyzz = (dz * dz - t3) * dy;
+        const float hxyz = (float)(dx * dy * dz);
+        const float U = Uf[0], V = Uf[1], W = Uf[2];
+        const float h3e = 13.5f * (hxxy * U * U * V + hxxz * U * U * W + hxyy * U * V * V + hyyz * V * V * W +
+                                   hxzz * U * W * W + hyzz * V * W * W) + 27.f * hxyz * U * V * W;
+        const float feqm1 = d + rho * (3.f * cu + 4.5f * cu * cu - 1.5f * uu + h3e);
+        // a^neq(Pi, u) of the fluid node
+        const float u = m[F_U], v = m[F_V], w = m[F_W];
+        const float pxx = m[F_XX], pxy = m[F_XY], pxz = m[F_XZ], pyy = m[F_YY], pyz = m[F_YZ], pzz = m[F_ZZ];
+        const float h2 = (dx * dx - t3) * pxx + (dy * dy - t3) * pyy + (dz * dz - t3) * pzz +
+                         2.f * (dx * dy * pxy + dx * dz * pxz + dy * dz * pyz);
+        const float an = 4.5f * h2 +
+                         13.5f * (hxxy * (2.f * u * pxy + v * pxx) + hxxz * (2.f * u * pxz + w * pxx) +
+                                  hxyy * (u * pyy + 2.f * v * pxy) + hyyz * (2.f * v * pyz + w * pyy) +
+                                  hxzz * (u * pzz + 2.f * w * pxz) + hyzz * (v * pzz + 2.f * w * pyz)) +
+                         27.f * hxyz * (u * pyz + v * pxz + w * pxy);
+        const float P = feqm1 + (1.f - omega) * an;
+        r.f = wq * P;
+        if (MODE == TSLB_MODE_COLOUR) {
+            const float dphi = phib - pht;
+            r.col += wq * fmaf(dphi, P, dphi);
+        } else if (MODE == TSLB_MODE_PHASEFIELD && c2 == 1) {
+            // g entering from the face (:984-986, :1044-1045)
+            const float eu = dx * Ub[0] + dy * Ub[1] + dz * Ub[2];
+            r.col += 0.125f * phib * (1.f + 3.f * eu);
+        }
+    }
+    return r;
+}
+
+// Half-way bounce-back off interior solid nodes, and off the faces of mask, all of
+// them bounce-back: first which of the 26 sources are solid (loads that wait on
+// nothing), then their reflected populations, added to acc.  As part of the general
+// path, direction by direction, a step of a 160 x 128 x 96 colour lattice with one
+// sphere / a packing of 300 took 373 / 1083 us and takes 179 / 466 us.
+template <int MODE, class Acc>
+__device__ __forceinline__ void bounce_solids(const StepArgs& a, const float* K, unsigned mask, int x, int y, int z, const Acc& acc) {
+    const int xm = x > 0 ? x - 1 : a.nx - 1, xp = x < a.nx - 1 ? x + 1 : 0;
+    unsigned from = 0;   // bit q: the source x - c of direction q is solid
+#pragma unroll 3
+    for (int r = 0; r < 9; ++r) {
+        int sy = y - (r % 3 - 1), sz = z - (r / 3 - 1);
+        sy = sy < 0 ? sy + a.ny : sy >= a.ny ? sy - a.ny : sy;
+        sz = sz < 0 ? sz + a.nz : sz >= a.nz ? sz - a.nz : sz;
+        const unsigned row = (unsigned)sz * a.plane + (unsigned)sy * a.nx;
+        const unsigned b = (bit_at(a.solid, row + xp) ? 1u : 0u) | (bit_at(a.solid, row + x) ? 2u : 0u) |
+                           (bit_at(a.solid, row + xm) ? 4u : 0u);
+        from |= b << 3 * r;
+    }
+    const unsigned behind = directions_behind(mask), zface = directions_behind(mask & 48u);
+    from |= behind;
+    float r[NACC];
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) r[i] = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < 27; ++q) {
+        if (!(from >> q & 1u)) continue;
+        const int dx = q % 3 - 1, dy = q / 3 % 3 - 1, dz = q / 9 - 1, c2 = dx * dx + dy * dy + dz * dz;
+        const float wq = wclass(c2);
+        acc_dir_rt(r, dx, dy, dz, wq * eval_P(K, 1, -dx, -dy, -dz));
+        const float b = -(dx * K[K_C1] + dy * K[K_C2] + dz * K[K_C3]);
+        // (colour: the reflected population carries the target's own colour; the pull
+        // visited a solid source as a node of phi 0, but no plane behind a z face)
+        if (MODE == TSLB_MODE_COLOUR) r[A_COL] += wq * ((zface >> q & 1u ? 0.f : K[K_C0]) + invlen(c2) * b);
+        if (MODE == TSLB_MODE_PHASEFIELD && c2 == 1) r[A_COL] += K[K_C0] + b;
+    }
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) acc[i] = r[i];
 }
 
 // ---- tile geometry ----
@@ -376,8 +434,8 @@ constexpr int ROWE = 40, MROW = ROWE * 4;   // elements, and bytes kept for a ro
 // nodes, [2][thread] (place, offset); the moments of populations from behind
 // faces, [NACC][thread]; sources of the chunk reads, [2][thread]; the phi ring;
 // phase field: the curvature work list (the candidate nodes' tile indices for
-// two planes, their curvatures, two counts).  What is used once a plane is
-// kept here rather than in registers.
+// two planes, their curvatures, two counts); the count of listed boundary nodes.
+// What is used once a plane is kept here rather than in registers.
 template <int MODE, int W>
 struct Smem {
     static constexpr int NT = 32 * W;
@@ -395,7 +453,8 @@ struct Smem {
     static constexpr int curv = ring + (MODE != TSLB_MODE_SINGLE ? RING * RAREA * 4 : 0);
     static constexpr int list = curv + (MODE == TSLB_MODE_PHASEFIELD ? NT * 4 : 0);
     static constexpr int count = list + (MODE == TSLB_MODE_PHASEFIELD ? 2 * NT * 2 : 0);
-    static constexpr int bytes = count + (MODE == TSLB_MODE_PHASEFIELD ? 16 : 0);
+    static constexpr int gcount = count + (MODE == TSLB_MODE_PHASEFIELD ? 16 : 0);
+    static constexpr int bytes = gcount + 16;
 };
 
 // gradient 3 sum_i p_i c_i phi(x+c_i) of one node (Ar1) or two (Ar2) from
@@ -591,11 +650,172 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// Coefficients, [coefficient][thread], and list of the nodes of plane s that take
+// the general boundary path, where the y values of plane s-1 were.
+template <int W>
+__device__ __forceinline__ float* listed_coefs(float4* exch, int s) {
+    return reinterpret_cast<float*>(exch + ((s + 1) & 1) * (2 * 3 * 32 * W));
+}
+template <int W>
+__device__ __forceinline__ int* listed(float* coefs) {
+    static_assert((NCOEF + 1) * 4 <= 2 * 3 * 16, "list and coefficients fit a plane's y values");
+    return reinterpret_cast<int*>(coefs + NCOEF * 32 * W);
+}
+// Moments of a node of the plane held in shared memory.
+template <int MODE, class T, int W>
+struct NodeMoments {
+    const StepArgs& a;
+    const char* m;
+    const float* phi;
+    // X0, y0, rx, mcol: the tile's first source column, first target row, ring column of
+    // its first phi column, byte of its first column in a row of moments (-1: node by node)
+    __device__ __forceinline__ NodeMoments(const StepArgs& a_, const char* sm, int row, int ln, int X0, int y0, int s, int rx, int mcol)
+        : a(a_) {
+        using SM = Smem<MODE, W>;
+        m = sm + SM::mom + (s & 1) * NMOM * W * MROW + row * MROW + (mcol >= 0 ? mcol + ln * (int)sizeof(T) : ln * 4);
+        if (sizeof(T) == 2 && mcol < 0) m += (((unsigned)s * a.plane + (unsigned)((y0 - 1 + row) * a.nx + X0 + ln)) & 1) * 2;
+        phi = reinterpret_cast<const float*>(sm + SM::ring) + (s & (RING - 1)) * SM::RAREA + (row + phi_rim(MODE)) * ROWE + rx + ln + phi_rim(MODE);
+    }
+    __device__ __forceinline__ float operator()(int f) const {
+        if (f == F_PHI) return MODE != TSLB_MODE_SINGLE ? *phi : 0.f;
+        return cvt_in<T>(*reinterpret_cast<const T*>(m + f * W * MROW), a, f);
+    }
+};
+
+// The listed nodes of plane s, half a warp a node, warp w taking entries 2 w,
+// 2 w + 2 W, ...; their sums go to the moments from behind faces.
+template <int MODE, class T, int W, bool TAU, bool SOLID>
+__device__ __forceinline__ void listed_nodes(const StepArgs& a, int X0, int y0, int s, int rx, int mcol, int cnt) {
+    using SM = Smem<MODE, W>;
+    constexpr int NT = 32 * W;
+    extern __shared__ float4 smem4[];
+    char* sm = reinterpret_cast<char*>(smem4);
+    float* coefs = listed_coefs<W>(reinterpret_cast<float4*>(sm + SM::exch), s);
+    const int* list = listed<W>(coefs);
+    const int lane = threadIdx.x, half = lane >> 4, hl = lane & 15;
+    const bool xper = a.face[0].kind == TSLB_BC_PERIODIC, yper = a.face[2].kind == TSLB_BC_PERIODIC, zper = a.face[4].kind == TSLB_BC_PERIODIC;
+    for (int e = 2 * threadIdx.y; e < cnt; e += 2 * W) {
+        const int tn = list[min(e + half, cnt - 1)], row = tn >> 5, ln = tn & 31, x = X0 + ln, y = y0 - 1 + row;
+        const unsigned mask = (xper ? 0u : (x == 0 ? 1u : 0u) | (x == a.nx - 1 ? 2u : 0u)) |
+                              (yper ? 0u : (y == 0 ? 4u : 0u) | (y == a.ny - 1 ? 8u : 0u)) |
+                              (zper ? 0u : (s == 0 ? 16u : 0u) | (s == a.nz - 1 ? 32u : 0u));
+        const NodeMoments<MODE, T, W> mom(a, sm, row, ln, X0, y0, s, rx, mcol);
+        const float dt = TAU ? reinterpret_cast<const float*>(sm + SM::dt)[(s & 1) * NT + tn] : 0.f;
+        // (beside interior solids any source may be one)
+        const unsigned dirs = SOLID ? 0x7ffffffu & ~(1u << 13) : directions_behind(mask);
+        const int nd = __popc(dirs);
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+#pragma unroll 1
+        for (int k = hl; k < nd; k += 16) {
+            const int q = nth_bit(dirs, k);
+            const Incoming in = direction_from_behind<MODE, T, SOLID>(a, coefs + tn, NT, mask, x, y, s, q, mom, dt);
+            acc_dir_rt(v, q % 3 - 1, q / 3 % 3 - 1, q / 9 - 1, in.f);
+            v[A_COL] += in.col;
+        }
+        __syncwarp();
+        // sums over the half warp: lanes that differ in bit h send each other the
+        // half of the values that the other keeps; lane hl is left with value hl
+#pragma unroll
+        for (int h = 8; h > 0; h >>= 1) {
+            const bool up = lane & h;
+#pragma unroll
+            for (int i = 0; i < h; ++i) {
+                const float keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+            }
+        }
+        if (hl < NACC && e + half < cnt) reinterpret_cast<float*>(sm + SM::bnd)[hl * NT + tn] = v[0];
+    }
+}
+
+// The populations entering this thread's node from behind one inlet or outlet
+// face f normal to y or z, where whole rows have one: the nine of them in turn, all
+// of a row at once.  160 x 128 x 96 colour steps with outlets normal to y / an inlet and
+// an outlet normal to z: 159 / 107 us (all 26 directions in turn 721 / 111).
+constexpr int IOFACE0 = 2;
+template <int MODE, class T, int W, bool TAU>
+__device__ __forceinline__ void io_face(const StepArgs& a, int X0, int y0, int s, int rx, int mcol, int f) {
+    using SM = Smem<MODE, W>;
+    constexpr int NT = 32 * W;
+    extern __shared__ float4 smem4[];
+    char* sm = reinterpret_cast<char*>(smem4);
+    const int lane = threadIdx.x, row = threadIdx.y, tid = row * 32 + lane, X = X0 + lane, Y = y0 - 1 + row;
+    const NodeMoments<MODE, T, W> mom(a, sm, row, lane, X0, y0, s, rx, mcol);
+    const float dt = TAU ? reinterpret_cast<const float*>(sm + SM::dt)[(s & 1) * NT + tid] : 0.f;
+    const FaceBC& fb = a.face[f];
+    const int ax = f >> 1, c = f & 1 ? -1 : 1;
+    const bool inlet = fb.kind == TSLB_BC_INLET, xper = a.face[0].kind == TSLB_BC_PERIODIC;
+    const bool pper = ax == 1 ? a.face[4].kind == TSLB_BC_PERIODIC : a.face[2].kind == TSLB_BC_PERIODIC;
+    float m[NF];
+#pragma unroll
+    for (int i = 0; i < NF; ++i) m[i] = mom(i);
+    float omega = a.omega_pf;
+    if (MODE == TSLB_MODE_COLOUR) {
+        const float ca = 0.5f * (1.f + m[F_PHI]), cb = 0.5f * (1.f - m[F_PHI]);
+        const float nu = 1.f / (ca * a.inv_nu_a + cb * a.inv_nu_b);
+        omega = 2.f / (6.f * nu + 1.f + 2.f * dt);
+    }
+    // rho at rest and (1 - omega) w a^neq(Pi, u); the moving part of f^eq is the ghost node's
+    float K[K_XYZ + 1];
+    coefs_moments(m[F_D], m, 0.f, 0.f, 0.f, 1.f - omega, K);
+    const float rho = 1.f + m[F_D], pht = m[F_PHI];
+    float v[NACC];
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) v[i] = 0.f;
+    // (colour mode: a source behind a y face was visited as a node of phi 0)
+    if (MODE == TSLB_MODE_COLOUR && ax < 2) v[A_COL] = (1.f / 6.f) * pht;
+    for (int q = 0; q < 9; ++q) {
+        // c along the face's normal, dx and dp (z of a y face, y of a z face) in its plane
+        const int dx = q % 3 - 1, dp = q / 3 - 1, dy = ax == 1 ? c : dp, dz = ax == 1 ? dp : c;
+        // the ghost node it leaves: periodic axes wrap, others clamp
+        const int np = ax == 1 ? a.nz : a.ny;
+        int gx = X - dx, gp = (ax == 1 ? s : Y) - dp;
+        gx = (unsigned)gx < (unsigned)a.nx ? gx : xper ? wrapi(gx, a.nx) : gx < 0 ? 0 : a.nx - 1;
+        gp = (unsigned)gp < (unsigned)np ? gp : pper ? wrapi(gp, np) : gp < 0 ? 0 : np - 1;
+        float U = fb.u[0], V = fb.u[1], Wv = fb.u[2], phib = m[F_PHI];
+        if (inlet) {
+            // the inlet plane's u, v, w, phi (boundary_cds_3D_module.f90:934-986)
+            const long long pa = plane_area(a, f), pi = (long long)gx + (long long)a.nx * gp;
+            U = __ldg(fb.plane + pi); V = __ldg(fb.plane + pa + pi); Wv = __ldg(fb.plane + 2 * pa + pi); phib = __ldg(fb.plane + 3 * pa + pi);
+        }
+        const float eu = dx * U + dy * V + dz * Wv;   // (g enters with the face's velocity)
+        if (!inlet) {
+            // zero gradient of the normal velocity (:992)
+            const float n = ld_field<T>(a, F_U + ax, ax == 1 ? nidx(a, gx, Y, gp) : nidx(a, gx, gp, s));
+            if (ax == 1) V = n;
+            else Wv = n;
+        }
+        const float t3 = 1.f / 3.f;
+        const float cu = dx * U + dy * V + dz * Wv, uu = U * U + V * V + Wv * Wv;
+        const float h3e = 13.5f * (U * V * ((dx * dx - t3) * dy * U + (dy * dy - t3) * dx * V) +
+                                   U * Wv * ((dx * dx - t3) * dz * U + (dz * dz - t3) * dx * Wv) +
+                                   V * Wv * ((dy * dy - t3) * dz * V + (dz * dz - t3) * dy * Wv)) +
+                          27.f * (float)(dx * dy * dz) * U * V * Wv;
+        const int c2 = 1 + dx * dx + dp * dp;
+        const float wq = wclass(c2), P = eval_P(K, 1, dx, dy, dz) + rho * (3.f * cu + 4.5f * cu * cu - 1.5f * uu + h3e);
+        acc_dir_rt(v, dx, dy, dz, wq * P);
+        if (MODE == TSLB_MODE_COLOUR) {
+            const float dphi = phib - pht;
+            v[A_COL] += wq * fmaf(dphi, P, dphi);
+        } else if (MODE == TSLB_MODE_PHASEFIELD && c2 == 1) {
+            v[A_COL] += 0.125f * phib * (1.f + 3.f * eu);
+        }
+    }
+    float* bnd = reinterpret_cast<float*>(sm + SM::bnd);
+#pragma unroll
+    for (int i = 0; i < NACC; ++i) bnd[i * NT + tid] = v[i];
+}
+
 // T: storage type of the moment state (float, __nv_bfloat16, __half).
 // One block's work: target planes z0 .. z1 - 1 of tile (bx, by) of lattice a.
 // TAU: the lattice has a per-node correction of the relaxation time (a.dtau).
 // SOLID: the lattice has interior solid nodes (bit masks a.solid, a.near).
-template <int MODE, class T, int W, bool TAU = false, bool SOLID = false>
+// GEN (a.general): 0 no node takes io_face or the general boundary path, 1 nodes take
+// io_face, 2 both; the plane loop of kernels without them is faster, as they cost it
+// registers (160 x 128 x 96 colour, 0 / 2: 93 / 98 us).
+template <int MODE, class T, int W, bool TAU, bool SOLID, int GEN>
 __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, int z0, int z1) {
     using A = Ar2;
     using F = Ar1;
@@ -616,6 +836,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     float* cq_curv = reinterpret_cast<float*>(sm + SM::curv);
     unsigned short* cq_list = reinterpret_cast<unsigned short*>(sm + SM::list);
     int* cq_n = reinterpret_cast<int*>(sm + SM::count);
+    int* gen_n = reinterpret_cast<int*>(sm + SM::gcount);
     const bool xper = a.face[0].kind == TSLB_BC_PERIODIC;
     const bool yper = a.face[2].kind == TSLB_BC_PERIODIC;
     const bool zper = a.face[4].kind == TSLB_BC_PERIODIC;
@@ -636,7 +857,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     // flags of the node: bits 0..3 the faces it touches (z faces are added per
     // plane), then: it, its lower, its upper neighbour lies behind an x or y
     // face; any node of the warp does
-    constexpr unsigned OUT0 = 64u, OUTD = 128u, OUTU = 256u, ANYOUT = 512u;
+    constexpr unsigned OUT0 = 64u, OUTD = 128u, OUTU = 256u, ANYOUT = 512u, GENXY = 1024u;
     unsigned fl = (n0.out ? OUT0 : 0u) | (nd.out ? OUTD : 0u) | (nu.out ? OUTU : 0u);
     if (!xper) fl |= (X == 0 ? 1u : 0u) | (X == a.nx - 1 ? 2u : 0u);
     if (!yper) fl |= (Y == 0 ? 4u : 0u) | (Y == a.ny - 1 ? 8u : 0u);
@@ -668,6 +889,9 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     // whose neighbours and reads ahead are planes of the lattice as they stand
     // take the iteration without those cases
     const bool inner = !SOLID && !a.xwrap && (xper || (X0 - RIM >= 0 && X0 + 32 + RIM <= a.nx)) && yin;
+
+    // the tile has nodes at an x or y face, which may take the general path (direction_from_behind)
+    if (GEN == 2 && ((!xper && (X0 <= 0 || X0 + 31 >= a.nx - 1)) || (!yper && (y0 == 0 || yend == a.ny)))) fl |= GENXY;
 
     // ---- phi ring: this thread fills its own node and up to NEX rim nodes ----
     const int rx = pchunks ? X0 - RIM - Xp : 0;   // ring column of the tile's first phi column
@@ -823,6 +1047,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         if (mom) {
             const unsigned zoff = (unsigned)(FAST ? z : zclamp(z)) * plane;
             const int par = (z & 1) * NMOM * W * MROW;
+            if (TAU) cp_async4(dts + (z & 1) * NT + tid, a.dtau + (zoff + n0.off));
             if (chunks) {
                 const T* src = srcs[0] + zoff;
                 if (lane < 30) {
@@ -840,7 +1065,6 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
                 for (int f = 0; f < NMOM; ++f)
                     cp_async4(st + f * W * MROW, static_cast<const unsigned*>(a.fi[f]) + (sizeof(T) == 4 ? id : id >> 1));
             }
-            if (TAU) cp_async4(dts + (z & 1) * NT + tid, a.dtau + (zoff + n0.off));
         }
         cp_async_commit();
     };
@@ -883,6 +1107,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         if (PHI && !ASYNC) phi_store(std::false_type{}, z, p);
     }
     if (PF && tid == 0) cq_n[0] = cq_n[1] = 0;
+    if (GEN == 2 && tid == 0) *gen_n = 0;
     cp_async_wait<0>();
     __syncthreads();
     // gradient so far at planes s (x, y: planes s-1 and s; z: their difference) and
@@ -934,6 +1159,10 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         // ---- 0. moments of the next plane, phi of the plane after the ring's last ----
         cp_async_wait<0>();
         __syncwarp();   // the warp's copies of the moments of plane s have landed
+        // The listed nodes' coefficients, [coefficient][thread], and the list are kept
+        // where the y values of plane s-1 were, once every warp has read those.
+        const bool gen = GEN == 2 && !FAST && s >= z0 && s < z1 && ((fl & GENXY) || (!zper && (s == 0 || s == a.nz - 1)));
+        if (gen) __syncthreads();
         PhiRow ph;
         if (more) load_ahead(fast, s + 1, s + 1 + RIM, wact, ph);
         // ---- curvatures of this plane's candidates, warp w taking entries w, w + nw, ...
@@ -1002,27 +1231,37 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
                 }
             }
             // ---- populations from behind non-periodic faces, target plane s ----
+            bool io = false;   // from behind one inlet or outlet face normal to y or z
             if (!FAST && s >= z0 && s < z1) {
                 const unsigned mask = (fl & 15u) | (zper ? 0u : (s == 0 ? 16u : 0u) | (s == a.nz - 1 ? 32u : 0u));
                 near = valid && (mask || (SOLID && bit_at(a.near, (unsigned)s * plane + n0.off)));
                 if (near) {
                     const Strided<NT> acc{bnd + tid};
-#pragma unroll
-                    for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
-                    bool bounce = (mask & mask >> 1 & 0x15u) == 0;   // (one face of each axis)
+                    bool allbounce = true;
 #pragma unroll
                     for (int f = 0; f < 6; ++f)
-                        if (mask >> f & 1u) bounce = bounce && a.face[f].kind == TSLB_BC_BOUNCEBACK;
+                        if (mask >> f & 1u) allbounce = allbounce && a.face[f].kind == TSLB_BC_BOUNCEBACK;
+                    const bool bounce = allbounce && (mask & mask >> 1 & 0x15u) == 0;   // (one face of each axis)
                     const int f = __ffs(mask) - 1, kind = f >= 0 ? a.face[f].kind : TSLB_BC_PERIODIC;
-                    if (SOLID && bit_at(a.near, (unsigned)s * plane + n0.off)) {
-                        boundary_target<MODE, T, TAU, SOLID>(a, K, mask, X, Y, s, acc);
-                    } else if (bounce) {
-                        bounce_target<MODE>(K, mask, acc);
-                    } else if ((mask & (mask - 1)) == 0 && (kind == TSLB_BC_VELOCITY || kind == TSLB_BC_PRESSURE)) {
-                        mom_take(s);
-                        face_target<MODE>(a, K, m, dt, f, acc);
-                    } else {
-                        boundary_target<MODE, T, TAU, SOLID>(a, K, mask, X, Y, s, acc);
+                    const bool solids = SOLID && bit_at(a.near, (unsigned)s * plane + n0.off);
+                    if (SOLID && solids && allbounce) {
+                        bounce_solids<MODE>(a, K, mask, X, Y, s, acc);
+                    } else if (!solids && (bounce || ((mask & (mask - 1)) == 0 && (kind == TSLB_BC_VELOCITY || kind == TSLB_BC_PRESSURE)))) {
+#pragma unroll
+                        for (int i = 0; i < NACC; ++i) acc[i] = 0.f;
+                        if (bounce) {
+                            bounce_target<MODE>(K, mask, acc);
+                        } else {
+                            mom_take(s);
+                            face_target<MODE>(a, K, m, dt, f, acc);
+                        }
+                    } else if (GEN && !solids && (mask & (mask - 1)) == 0 && f >= IOFACE0) {
+                        io = true;   // (taken when the coefficients' registers are free)
+                    } else if (GEN == 2) {
+                        float* gen_k = listed_coefs<W>(exch, s);
+                        listed<W>(gen_k)[atomicAdd(gen_n, 1)] = tid;
+#pragma unroll
+                        for (int c = 0; c < NCOEF; ++c) gen_k[c * NT + tid] = K[c];
                     }
                 }
             }
@@ -1127,6 +1366,10 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
                 }
                 send(2, j0.td, cc, t, c);
             }
+            if (GEN && !FAST && io) {
+                const int f = (fl & 15u) ? __ffs(fl & 15u) - 1 : s == 0 ? 4 : 5;
+                io_face<MODE, T, W, TAU>(a, X0, y0, s, rx, chunks ? (X0 - Xm) * (int)sizeof(T) : -1, f);
+            }
         }
         // phase field: candidates of the next source plane (its phi is staged)
         if (PF) {
@@ -1136,6 +1379,15 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         if (PHI && !ASYNC && more) phi_store(fast, s + 1 + RIM, ph);
         cp_async_wait<1>();   // this thread's phi copies have landed
         __syncthreads();
+        if (gen) {   // the listed nodes
+            const int cnt = *gen_n;
+            if (cnt > 0) {
+                listed_nodes<MODE, T, W, TAU, SOLID>(a, X0, y0, s, rx, chunks ? (X0 - Xm) * (int)sizeof(T) : -1, cnt);
+                __syncthreads();
+                // (the next entries come after a barrier that follows this)
+                if (tid == 0) *gen_n = 0;
+            }
+        }
         if (!wtgt) return;
         // ---- 3. y and z sums ----
         V2 HA[3], HB[3], HM[3];
@@ -1232,7 +1484,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
 // tile.  zchunk = 0: the tiles of one x position, each with all its target
 // planes, are a sequence of planes; grid / tx blocks take equal shares of it,
 // in one piece or, across the end of a tile, in several.
-template <int MODE, class T, int W, bool TAU = false, bool SOLID = false>
+template <int MODE, class T, int W, bool TAU, bool SOLID, int GEN>
 __global__ void __launch_bounds__(32 * W, BIGW / W) step_kernel(const __grid_constant__ StepArgs a) {
     cudaTriggerProgrammaticLaunchCompletion();   // the next step may start; it waits as this one does
     const int planes = a.zt1 - a.zt0, tx = a.xwrap ? 1 : (a.nx + LXV - 1) / LXV, ty = (a.ny + a.th - 1) / a.th;
@@ -1249,7 +1501,7 @@ __global__ void __launch_bounds__(32 * W, BIGW / W) step_kernel(const __grid_con
     }
     while (p < end) {
         const int by = p / planes, z = p % planes, n = min(end - p, planes - z);
-        step_block<MODE, T, W, TAU, SOLID>(a, bx, by, a.zt0 + z, a.zt0 + z + n);
+        step_block<MODE, T, W, TAU, SOLID, GEN>(a, bx, by, a.zt0 + z, a.zt0 + z + n);
         p += n;
         if (p < end) __syncthreads();
     }
@@ -1271,7 +1523,7 @@ struct WorkItem {
 // ticket and step[2] the work counter: the last block of the launch to
 // finish, after every block has read the step and taken its last item,
 // advances the step and clears the other two for the next launch.
-template <int MODE, class T>
+template <int MODE, class T, int GEN>
 __global__ void __launch_bounds__(32 * SMALLW, BIGW / SMALLW) ensemble_kernel(const StepArgs* __restrict__ args,
                                                           const WorkItem* __restrict__ work, int nwork,
                                                           unsigned int* step) {
@@ -1289,7 +1541,7 @@ __global__ void __launch_bounds__(32 * SMALLW, BIGW / SMALLW) ensemble_kernel(co
             __syncthreads();
             cur = w.dom;
         }
-        step_block<MODE, T, SMALLW>(sa, w.bx, w.by, sa.zt0 + w.bz * sa.zchunk, min(sa.zt0 + (w.bz + 1) * sa.zchunk, sa.zt1));
+        step_block<MODE, T, SMALLW, false, false, GEN>(sa, w.bx, w.by, sa.zt0 + w.bz * sa.zchunk, min(sa.zt0 + (w.bz + 1) * sa.zchunk, sa.zt1));
         __syncthreads();
         // every thread has read `next` (it was read before this item's barriers)
         if (step) {
