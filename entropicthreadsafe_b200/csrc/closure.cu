@@ -103,7 +103,10 @@ __global__ void image_kernel(const float* __restrict__ params, Image* img) {
 // Shared-memory prologue of the MLP kernels: mbarrier, TMEM, the image copy.
 // The training kernel is launched while the optimiser of the step before may
 // still be writing the image (train_pass): `before` runs first, then the
-// kernel waits for that step, and only then is the image read.
+// kernel waits for that step, and only then is the image read.  The inference
+// kernel copies it first: behind the set-up, as for training, it cost the kernel
+// 48 bytes of spills more a thread and a refresh of the 192 x 192 x 384 jet
+// @A@ us instead of @B@.
 struct Smem {
     Image* im;
     uint4* act;
@@ -114,9 +117,8 @@ struct Smem {
     float* red;
 };
 
-template <class Before>
-__device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int off_misc, bool train, uint32_t ncols,
-                                           Before before) {
+template <bool TRAIN, class Before>
+__device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int off_misc, uint32_t ncols, Before before) {
     Smem S;
     S.im = reinterpret_cast<Image*>(sm);
     S.act = reinterpret_cast<uint4*>(sm + OFF_ACT);
@@ -126,7 +128,11 @@ __device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int o
     S.abort_s = reinterpret_cast<int*>(sm + off_misc + 12);
     S.red = reinterpret_cast<float*>(sm + off_misc + 64);
     const int tid = threadIdx.x;
-    if (train) {
+    const uint4* src = reinterpret_cast<const uint4*>(gimg);
+    uint4* dst = reinterpret_cast<uint4*>(sm);
+    if (!TRAIN)
+        for (int i = tid; i < IMG16; i += TILE) dst[i] = src[i];
+    if (TRAIN) {
         // constant chunks of ACT: a 1 in the first column of chunk 10, zeros in chunk 11
         const float one[8] = {1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         S.act[act_chunk(tid, 10)] = pack8(one);
@@ -138,15 +144,13 @@ __device__ __forceinline__ Smem smem_setup(uint8_t* sm, const Image* gimg, int o
     }
     if ((tid >> 5) == 0) tc::tmem_alloc(S.tslot, ncols);
     before();
-    if (train) {
+    if (TRAIN) {
         cudaGridDependencySynchronize();
         cudaTriggerProgrammaticLaunchCompletion();
-    }
-    const uint4* src = reinterpret_cast<const uint4*>(gimg);
-    uint4* dst = reinterpret_cast<uint4*>(sm);
 #pragma unroll
-    for (int k = 0; k < (IMG16 + TILE - 1) / TILE; ++k)
-        if (tid + k * TILE < IMG16) dst[tid + k * TILE] = src[tid + k * TILE];
+        for (int k = 0; k < (IMG16 + TILE - 1) / TILE; ++k)
+            if (tid + k * TILE < IMG16) dst[tid + k * TILE] = src[tid + k * TILE];
+    }
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -257,7 +261,7 @@ template <class Src>
 __global__ void __launch_bounds__(TILE, 6) infer_kernel(const Image* __restrict__ gimg, Src src, long long n,
                                                         unsigned int* gflag) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    Smem S = smem_setup(sm, gimg, OFF_MISC_INFER, false, 64, [] {});
+    Smem S = smem_setup<false>(sm, gimg, OFF_MISC_INFER, 64, [] {});
     const uint32_t tb = *S.tslot;
     const Image& im = *S.im;
     const int tid = threadIdx.x;
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(TILE, 1) train_kernel(const TrainArgs a) {
         row.tg = valid ? a.tgt[idx] : 0.f;
         row.wg = valid ? a.wgt[idx] : 0.f;
     };
-    Smem S = smem_setup(sm, a.img, OFF_MISC_TRAIN, true, 256, [&] { load_row(blockIdx.x); });
+    Smem S = smem_setup<true>(sm, a.img, OFF_MISC_TRAIN, 256, [&] { load_row(blockIdx.x); });
     const uint32_t tb = *S.tslot;
     const Image& im = *S.im;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
