@@ -105,8 +105,8 @@ __global__ void image_kernel(const float* __restrict__ params, Image* img) {
 // still be writing the image (train_pass): `before` runs first, then the
 // kernel waits for that step, and only then is the image read.  The inference
 // kernel copies it first: behind the set-up, as for training, it cost the kernel
-// 48 bytes of spills more a thread and a refresh of the 192 x 192 x 384 jet
-// @A@ us instead of @B@.
+// 48 bytes of spills more a thread, and a refresh of a 192 x 192 x 384 lattice
+// 685 us instead of 579.
 struct Smem {
     Image* im;
     uint4* act;
