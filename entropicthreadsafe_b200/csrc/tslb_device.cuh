@@ -130,6 +130,8 @@ __host__ __device__ inline float rand_noseeded(int i, int j, int k, int l) {
     return uni;
 }
 
+// bit i of a mask (set before any step that reads it is launched, so the read-only
+// path is open to it, as to nothing else that a step reads)
 __device__ __forceinline__ bool bit_at(const unsigned int* b, long long i) {
     return (__ldg(b + (i >> 5)) >> (i & 31)) & 1u;
 }
@@ -284,7 +286,7 @@ __device__ float phi_at(const StepArgs& a, int x, int y, int z) {
     }
     if (face < 0) return ld_field<T>(a, F_PHI, nidx(a, c[0], c[1], c[2]));
     const FaceBC& fb = a.face[face];
-    if (fb.kind == TSLB_BC_INLET) return __ldg(fb.plane + 3 * plane_area(a, face) + plane_index(a, face, c[0], c[1], c[2]));
+    if (fb.kind == TSLB_BC_INLET) return fb.plane[3 * plane_area(a, face) + plane_index(a, face, c[0], c[1], c[2])];
     if (a.wall_phi_mode == 0) return fb.phi;
     return ld_field<T>(a, F_PHI, nidx(a, c[0], c[1], c[2]));
 }

@@ -309,10 +309,10 @@ __device__ __forceinline__ Incoming direction_from_behind(const StepArgs& a, con
             // the inlet plane at the ghost node (boundary_cds_3D_module.f90:934-986:
             // u, v, w of node (i, j, 1) feed the populations it sends)
             const long long pa = plane_area(a, vface), pi = plane_index(a, vface, g[0], g[1], g[2]);
-            Ub[0] = __ldg(fb.plane + pi);
-            Ub[1] = __ldg(fb.plane + pa + pi);
-            Ub[2] = __ldg(fb.plane + 2 * pa + pi);
-            phib = __ldg(fb.plane + 3 * pa + pi);
+            Ub[0] = fb.plane[pi];
+            Ub[1] = fb.plane[pa + pi];
+            Ub[2] = fb.plane[2 * pa + pi];
+            phib = fb.plane[3 * pa + pi];
         } else if (fb.kind == TSLB_BC_OUTLET || fb.kind == TSLB_BC_PRESSURE) {
             phib = m[F_PHI];
         }
@@ -778,7 +778,7 @@ __device__ __forceinline__ void io_face(const StepArgs& a, int X0, int y0, int s
         if (inlet) {
             // the inlet plane's u, v, w, phi (boundary_cds_3D_module.f90:934-986)
             const long long pa = plane_area(a, f), pi = (long long)gx + (long long)a.nx * gp;
-            U = __ldg(fb.plane + pi); V = __ldg(fb.plane + pa + pi); Wv = __ldg(fb.plane + 2 * pa + pi); phib = __ldg(fb.plane + 3 * pa + pi);
+            U = fb.plane[pi]; V = fb.plane[pa + pi]; Wv = fb.plane[2 * pa + pi]; phib = fb.plane[3 * pa + pi];
         }
         const float eu = dx * U + dy * V + dz * Wv;   // (g enters with the face's velocity)
         if (!inlet) {
