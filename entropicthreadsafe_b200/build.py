@@ -21,7 +21,7 @@ OUT = os.path.join(HERE, "libtslb.so")
 DRIVER_SRC = os.path.join(HERE, "driver", "tslb_run.cpp")
 DRIVER = os.path.join(HERE, "tslb_run")
 SOURCES = ["tslb.cu", "k_scalar.cu", "k_inlet.cu", "k_general.cu", "closure.cu", "tslb_io.cpp"]
-HEADERS = ["tslb_device.cuh", "tslb_step.cuh", "step_launch.h", "step_variants.cuh", "tslb_internal.h", "tcgen05.cuh", "closure_mlp.cuh"]
+HEADERS = ["tslb_device.cuh", "tslb_step.cuh", "step_launch.h", "step_variants.cuh", "step_plan.h", "tslb_internal.h", "tcgen05.cuh", "closure_mlp.cuh"]
 INCLUDES = ["tslb.h", "tslb_closure.h", "tslb_io.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -682,69 +682,24 @@ int ensure_normals(tslb_ctx* c) {
     return TSLB_OK;
 }
 
-// How the step kernel cuts a lattice: warps of a block, target rows of a tile,
-// target planes of a block (0: `grid` blocks share the tiles' planes equally).
-struct StepPlan { int warps, th, zchunk, grid; };
 constexpr int kEnsBlocksPerSM = BIGW / SMALLW;   // ensemble blocks (SMALLW warps) resident on an SM
-
-int even_rows(int ny, int most) {   // tiles of equal height, at most `most` rows (any positive number)
-    most = std::min(most, ny);
-    const int tiles = (int)(((long long)ny + most - 1) / most);
-    return (int)(((long long)ny + tiles - 1) / tiles);
-}
 
 // some tiles' boundary nodes make all their planes slower than other tiles'
 bool slow_columns(const tslb_params& p, int nx, int ny, int nz, bool solids) {
     return general_nodes(p, nx, ny, nz, solids) && (p.bc[0] != TSLB_BC_PERIODIC || p.bc[2] != TSLB_BC_PERIODIC);
 }
 
-// The plan with the least estimated time, about microseconds on a B200.  A block
-// takes `plane` per source plane and about `extra` planes' time outside its
-// target planes (two more source planes, its start); blocks run in waves.
-// Measured on the 384 x 192 x 128 colour channel: 16-warp blocks in 32 / 16 / 8
-// plane chunks 0.333 / 0.355 / 0.404 ms, 8-warp blocks in 64 / 32 / 16 plane
-// chunks 0.331 / 0.340 / 0.352 ms: 3 planes extra, and a plane of two 8-warp
-// blocks on an SM takes 0.85 of one of 16 warps, with fewer rows (6 of 8 are
-// targets, against 14 of 16).  Equal shares have no last wave, but their blocks
-// are at different planes and share less of what they read: 8% slower a plane
-// (48 against 51 us in the best chunks on a 173 x 59 x 91 Couette cell).  The phase field takes chunks only, and short
-// ones: planes with interface nodes are about three times slower, so the last
-// blocks to finish are those across a droplet, by their length (96^3 with one
-// droplet: 130 us in 24-plane chunks).  So do lattices with interior solids or with
-// nodes on the general boundary path at x or y faces, whose tiles are the slow ones.
-StepPlan step_plan(int nx, int ny, int nz, const tslb_params& p, bool solids, int sms) {
-    StepPlan best{BIGW, 1, nz, 0};
-    double least = 1e300;
-    const bool xper = p.bc[0] == TSLB_BC_PERIODIC, uneven = p.mode == TSLB_MODE_PHASEFIELD || solids || slow_columns(p, nx, ny, nz, solids);
-    const long long tx = (xper && nx <= 32) ? 1 : (nx + LXV - 1) / LXV;
-    constexpr double extra = 3.0;
-    for (int w : {BIGW, SMALLW}) {
-        const int th = even_rows(ny, w - 2), bps = BIGW / w;
-        const long long ty = (ny + th - 1) / th, slots = (long long)bps * sms;
-        auto plane = [&](long long blocks) { return w == BIGW ? 2.0 : blocks <= sms ? 1.25 : 1.72; };
-        for (int nc = 1; nc <= nz; ++nc) {
-            const int zc = (nz + nc - 1) / nc;
-            const long long blocks = tx * ty * ((nz + zc - 1) / zc);
-            const double tail = uneven ? 3.0 * zc : 0.0;
-            const double cost = (double)((blocks + slots - 1) / slots) * (zc + extra) * plane(blocks) + tail;
-            if (cost < least) { least = cost; best = StepPlan{w, th, zc, 0}; }
-            if (nc > 1 && blocks > 16 * slots) break;   // more waves only add planes outside the chunks
-        }
-        const long long parts = std::min(slots / tx, ty * nz);
-        if (!uneven && parts > 0 && ty * nz < (1LL << 31)) {
-            const double share = (double)(ty * nz) / parts;
-            const double cost = 1.08 * (share + extra * (share / nz + 1.0)) * plane(parts * tx);
-            if (cost < least) { least = cost; best = StepPlan{w, th, 0, (int)(parts * tx)}; }
-        }
-    }
-    return best;
+// The plan of a step of nz planes (step_plan.h).
+StepPlan plan_of(const tslb_params& p, int nx, int ny, int nz, bool solids, int sms) {
+    const bool uneven = p.mode == TSLB_MODE_PHASEFIELD || solids || slow_columns(p, nx, ny, nz, solids);
+    return step_plan(nx, ny, nz, p.bc[0] == TSLB_BC_PERIODIC, uneven, sms);
 }
 
 // The plan of a context's step, for the planes it updates and its solid nodes.
 void plan_step(tslb_ctx* c) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const StepPlan plan = step_plan(c->nx, c->ny, (c->zt1 > 0 ? c->zt1 : c->nz) - c->zt0, c->p, c->solid_on, sms);
+    const StepPlan plan = plan_of(c->p, c->nx, c->ny, (c->zt1 > 0 ? c->zt1 : c->nz) - c->zt0, c->solid_on, sms);
     c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
 }
 
@@ -1622,7 +1577,7 @@ extern "C" int tslb_step_noalloc(const tslb_params* p, int nx, int ny, int nz, c
     for (int f = 0; f < NF; ++f) view.scale[f] = 1.0f;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const StepPlan plan = step_plan(nx, ny, nz, *p, false, sms);
+    const StepPlan plan = plan_of(*p, nx, ny, nz, false, sms);
     view.warps = plan.warps; view.th = plan.th; view.zchunk = plan.zchunk; view.grid = plan.grid;
     StepArgs a = make_args(&view, d_in, d_out);
     if ((e = launch_step_kernel(a, p->mode, TSLB_PREC_FP32, st, true, true)) != cudaSuccess)

@@ -49,6 +49,7 @@
 // slower still (0.66 ms).
 #pragma once
 
+#include "step_plan.h"
 #include "tslb_device.cuh"
 
 namespace tslb {
@@ -409,11 +410,7 @@ __device__ __forceinline__ void bounce_solids(const StepArgs& a, const float* K,
     for (int i = 0; i < NACC; ++i) acc[i] = r[i];
 }
 
-// ---- tile geometry ----
-constexpr int LXV = 30;       // target columns of a warp: lanes 1 .. 30 (lanes 0 and 31 are sources only)
-// Warps of a block, W: 16 (one block on an SM) or 8 (two, for lattices whose
-// rows or planes do not fill 16).
-constexpr int BIGW = 16, SMALLW = 8;
+// ---- tile geometry (LXV, BIGW, SMALLW: step_plan.h) ----
 constexpr int NMOM = NF - 1;  // moments read per node (phi comes from the phi ring)
 
 // Phi rows and columns held beyond the block's source nodes: colour mode
