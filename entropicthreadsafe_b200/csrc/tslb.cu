@@ -95,7 +95,7 @@ int general_nodes(const tslb_params& p, int nx, int ny, int nz, bool solids) {
     for (int f = 0; f < 6; ++f) {
         const int k = p.bc[f];
         if (k == TSLB_BC_PERIODIC) continue;
-        axes += f & 1;
+        axes += !(f & 1) || p.bc[f - 1] == TSLB_BC_PERIODIC;   // (once an axis)
         const bool through = k == TSLB_BC_INLET || k == TSLB_BC_OUTLET;
         io = io || through;
         xio = xio || (through && f < 2);
@@ -103,6 +103,15 @@ int general_nodes(const tslb_params& p, int nx, int ny, int nz, bool solids) {
         thin = thin || (f < 2 ? nx : f < 4 ? ny : nz) == 1;
     }
     return xio || thin || (!bounce && (axes > 1 || (axes > 0 && solids))) ? 2 : io ? 1 : 0;
+}
+
+// The parameters with the faces a step meets: a slab's halo sides are none (their
+// boundary kinds are placeholders).
+tslb_params faces_met(const tslb_ctx* c) {
+    tslb_params p = c->p;
+    if (c->halo_lo) p.bc[4] = TSLB_BC_PERIODIC;
+    if (c->halo_hi) p.bc[5] = TSLB_BC_PERIODIC;
+    return p;
 }
 
 StepArgs make_args(tslb_ctx* c, const void* in, void* out) {
@@ -144,7 +153,7 @@ StepArgs make_args(tslb_ctx* c, const void* in, void* out) {
     a.dtau = c->closure ? c->dtau : (c->base_on ? c->dtau_base : nullptr);
     a.solid = c->solid_on ? c->solid : nullptr;
     a.near = c->solid_on ? c->near : nullptr;
-    a.general = general_nodes(c->p, c->nx, c->ny, c->nz, c->solid_on);
+    a.general = general_nodes(faces_met(c), c->nx, c->ny, c->nz, c->solid_on);
     a.sr = 1;
     a.sr_step = (unsigned int)c->steps_done;
     a.sr_counter = nullptr;
@@ -699,7 +708,7 @@ StepPlan plan_of(const tslb_params& p, int nx, int ny, int nz, bool solids, int 
 void plan_step(tslb_ctx* c) {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const StepPlan plan = plan_of(c->p, c->nx, c->ny, (c->zt1 > 0 ? c->zt1 : c->nz) - c->zt0, c->solid_on, sms);
+    const StepPlan plan = plan_of(faces_met(c), c->nx, c->ny, (c->zt1 > 0 ? c->zt1 : c->nz) - c->zt0, c->solid_on, sms);
     c->warps = plan.warps; c->th = plan.th; c->zchunk = plan.zchunk; c->grid = plan.grid;
 }
 
@@ -1723,6 +1732,12 @@ int tslb_create_slab(const tslb_params* p, int nx, int ny, int nz, int z_begin, 
     c->zt0 = lo;
     c->zt1 = lo + (z_end - z_begin);
     plan_step(c);
+    rc = tslb_internal::prepare_step_kernel(c);
+    if (rc) {
+        g_create_error = c->err;
+        tslb_destroy(c);
+        return rc;
+    }
     *out = c;
     return TSLB_OK;
 }
