@@ -84,6 +84,17 @@ int validate(const tslb_params* p, int nx, int ny, int nz, std::string& why) {
     return TSLB_OK;
 }
 
+// The step counts a lattice's nodes in unsigned 32-bit numbers and the columns of a
+// plane, and planes and coordinates a tile beyond the lattice, in int.  A slab of a
+// larger lattice is measured by its own planes.
+int indexable(int nx, int ny, int nz, std::string& why) {
+    constexpr long long margin = 1024;
+    if ((long long)nx * ny <= (1LL << 31) - margin && nz <= (1LL << 31) - margin && (long long)nx * ny * nz <= (1LL << 32) - margin)
+        return TSLB_OK;
+    why = "lattice too large: at most 2^31 - 1024 nodes in a plane and 2^32 - 1024 in all (on one device)";
+    return TSLB_ERR_ARG;
+}
+
 // Which nodes of a lattice have no closed sums of the populations from behind their
 // faces (StepArgs::general): 1 those at one inlet or outlet face normal to y or z;
 // 2 also those at inlets and outlets normal to x, at edges that are not all
@@ -880,6 +891,7 @@ int tslb_create(const tslb_params* p, int nx, int ny, int nz, tslb_ctx** out) {
     *out = nullptr;
     std::string why;
     int rc = validate(p, nx, ny, nz, why);
+    if (!rc) rc = indexable(nx, ny, nz, why);
     if (rc) return fail(nullptr, rc, why);
     tslb_ctx* c = new (std::nothrow) tslb_ctx();
     if (!c) return fail(nullptr, TSLB_ERR_ARG, "out of host memory");
@@ -1551,6 +1563,7 @@ extern "C" int tslb_step_noalloc(const tslb_params* p, int nx, int ny, int nz, c
                                  long long field_stride, void* stream) {
     std::string why;
     int rc = validate(p, nx, ny, nz, why);
+    if (!rc) rc = indexable(nx, ny, nz, why);
     if (rc) return noalloc_fail(rc, "tslb_step_noalloc: " + why);
     const long long n = (long long)nx * ny * nz;
     if (!d_in || !d_out) return noalloc_fail(TSLB_ERR_ARG, "tslb_step_noalloc: NULL device buffer");

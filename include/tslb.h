@@ -141,7 +141,9 @@ typedef struct tslb_ctx tslb_ctx;
 void tslb_default_params(tslb_params* p);
 
 /* Validate *p and the sizes, allocate the device state of nx*ny*nz nodes
- * and a CUDA stream on the current device.  *out is NULL on failure. */
+ * and a CUDA stream on the current device.  *out is NULL on failure.  A
+ * lattice (of slabs: each slab) has at most 2^31 - 1024 nodes in an x-y plane
+ * and 2^32 - 1024 in all; more is TSLB_ERR_ARG. */
 int  tslb_create(const tslb_params* p, int nx, int ny, int nz, tslb_ctx** out);
 void tslb_destroy(tslb_ctx* ctx);
 
