@@ -873,11 +873,12 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     };
 
     // ---- rows read as 16-byte chunks: FP32 or 16-bit rows of whole chunks (nx a
-    // multiple of EPC), the tile's columns (with the phi rim) inside a row ----
+    // multiple of EPC), x periodic (every chunk is wrapped whole) or the tile's
+    // columns (with the phi rim) inside a row ----
     constexpr int EPC = 16 / (int)sizeof(T), CPR = ROWE / EPC;   // elements of a chunk, chunks of a row
     const int X0 = X - lane;
     const int Xm = X0 & ~(EPC - 1), Xp = (X0 - RIM) & ~3;        // first columns read (moments, phi)
-    const bool chunks = !a.xwrap && a.nx % EPC == 0 && X0 - RIM >= 0 && max(Xm, Xp) + ROWE <= a.nx;
+    const bool chunks = a.nx % EPC == 0 && (xper || (X0 - RIM >= 0 && max(Xm, Xp) + ROWE <= a.nx));
     const bool yin = yper || (y0 - 1 - RIM >= 0 && y0 - 1 + W + RIM <= a.ny);   // no row behind a y face
     // (a tile with computed ghost rows reads phi node by node in every warp: a rim
     // node belongs to another warp than the row it ends, so a block reads in one way)
@@ -968,7 +969,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
     // one, a rim row (cpp).
     constexpr int FPI = 30 / CPR, NCHK = (NMOM + FPI - 1) / FPI, mlast = CPR * (NMOM - FPI * (NCHK - 1));
     const T** srcs = reinterpret_cast<const T**>(sm + SM::src) + tid;   // kept in shared memory: moments, phi
-    srcs[0] = static_cast<const T*>(a.in) + (lane / CPR) * a.N + (n0.off - X + Xm + (lane % CPR) * EPC);
+    srcs[0] = static_cast<const T*>(a.in) + (lane / CPR) * a.N + (xy_node(a, 0, Y, xper, yper).off + wrapi(Xm + (lane % CPR) * EPC, a.nx));
     char* cpd = mst + (lane / CPR) * W * MROW + wy * MROW + (lane % CPR) * 16;
     const T* cpp = nullptr;
     int cpr = 0;
@@ -981,7 +982,7 @@ __device__ __forceinline__ void step_block(const StepArgs& a, int bx, int by, in
         }
         if (has) {
             const XYNode n = xy_node(a, 0, y0 - 1 + r - RIM, xper, yper);
-            cpp = phin + (n.off + Xp + (lane % 10) * 4);
+            cpp = phin + (n.off + wrapi(Xp + (lane % 10) * 4, a.nx));
             cpr = r * RW + (lane % 10) * 4;
         }
     }
