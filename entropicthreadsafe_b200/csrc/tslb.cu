@@ -711,8 +711,11 @@ bool slow_columns(const tslb_params& p, int nx, int ny, int nz, bool solids) {
 
 // The plan of a step of nz planes (step_plan.h).
 StepPlan plan_of(const tslb_params& p, int nx, int ny, int nz, bool solids, int sms) {
-    const bool uneven = p.mode == TSLB_MODE_PHASEFIELD || solids || slow_columns(p, nx, ny, nz, solids);
-    return step_plan(nx, ny, nz, p.bc[0] == TSLB_BC_PERIODIC, uneven, sms);
+    const PlanCosts& costs = solids || slow_columns(p, nx, ny, nz, solids) ? kUnevenCosts
+                             : p.mode == TSLB_MODE_PHASEFIELD              ? kPhaseCosts
+                             : p.precision == TSLB_PREC_FP32               ? kEvenCosts
+                                                                           : kEven16Costs;
+    return step_plan(nx, ny, nz, p.bc[0] == TSLB_BC_PERIODIC, costs, sms);
 }
 
 // The plan of a context's step, for the planes it updates and its solid nodes.

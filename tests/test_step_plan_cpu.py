@@ -15,26 +15,25 @@ SOURCE = r"""
 #include <cstdio>
 #include <random>
 using namespace tslb;
-static StepPlan full(int nx, int ny, int nz, bool xper, bool uneven, int sms) {
+static StepPlan full(int nx, int ny, int nz, bool xper, const PlanCosts& costs, int sms) {
     StepPlan best{BIGW, 1, nz, 0};
     double least = 1e300;
     const long long tx = (xper && nx <= 32) ? 1 : (nx + LXV - 1LL) / LXV;
     for (int w : {BIGW, SMALLW}) {
         const int th = even_rows(ny, w - 2), bps = BIGW / w;
         const long long ty = (ny + th - 1LL) / th, slots = (long long)bps * sms;
-        auto plane = [&](long long blocks) { return w == BIGW ? 2.0 : blocks <= sms ? 1.25 : 1.72; };
+        auto plane = [&](long long blocks) { return w == BIGW ? 2.0 : blocks <= sms ? costs.one : costs.two; };
         for (int nc = 1; nc <= nz; ++nc) {
             const int zc = (nz + nc - 1) / nc;
             const long long blocks = tx * ty * ((nz + zc - 1) / zc);
-            const double tail = uneven ? 3.0 * zc : 0.0;
-            const double cost = (double)((blocks + slots - 1) / slots) * (zc + 3.0) * plane(blocks) + tail;
+            const double cost = (double)((blocks + slots - 1) / slots) * (zc + 3.0) * plane(blocks) + costs.tail * zc;
             if (cost < least) { least = cost; best = StepPlan{w, th, zc, 0}; }
             if (nc > 1 && blocks > 16 * slots) break;
         }
         const long long parts = std::min(slots / tx, ty * nz);
-        if (!uneven && parts > 0 && ty * nz < (1LL << 31)) {
+        if (costs.tail == 0.0 && parts > 0 && ty * nz < (1LL << 31)) {
             const double share = (double)(ty * nz) / parts;
-            const double cost = 1.08 * (share + 3.0 * (share / nz + 1.0)) * plane(parts * tx);
+            const double cost = costs.share * (share + 3.0 * (share / nz + 1.0)) * plane(parts * tx);
             if (cost < least) { least = cost; best = StepPlan{w, th, 0, (int)(parts * tx)}; }
         }
     }
@@ -46,7 +45,7 @@ static double time_of(F f) {
     for (int r = 0; r < 7; ++r) {
         const auto t0 = std::chrono::steady_clock::now();
         volatile int sink = 0;
-        for (int i = 0; i < 200; ++i) sink = sink + f(16, 16, 4096 + (i & 1), true, false, 148).zchunk;
+        for (int i = 0; i < 200; ++i) sink = sink + f(16, 16, 4096 + (i & 1), true, kEvenCosts, 148).zchunk;
         best = std::min(best, std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
     }
     return best;
@@ -58,10 +57,11 @@ int main() {
     for (int i = 0; i < 20000; ++i) {
         const int top = i % 4 == 0 ? 40 : i % 4 == 1 ? 400 : 5000;
         const int nx = size(top), ny = size(top), nz = size(i % 7 == 0 ? 60000 : top), sms = i % 5 ? 148 : 1 + size(200);
-        const bool xper = rng() & 1, uneven = rng() & 1;
-        const StepPlan a = step_plan(nx, ny, nz, xper, uneven, sms), b = full(nx, ny, nz, xper, uneven, sms);
+        const bool xper = rng() & 1;
+        const PlanCosts all[4] = {kEvenCosts, kEven16Costs, kPhaseCosts, kUnevenCosts}, costs = all[rng() % 4];
+        const StepPlan a = step_plan(nx, ny, nz, xper, costs, sms), b = full(nx, ny, nz, xper, costs, sms);
         if (a.warps != b.warps || a.th != b.th || a.zchunk != b.zchunk || a.grid != b.grid) {
-            if (bad++ < 5) std::printf("%d x %d x %d %d %d %d: %d %d %d %d, full search %d %d %d %d\n", nx, ny, nz, xper, uneven, sms,
+            if (bad++ < 5) std::printf("%d x %d x %d %d %.2f %d: %d %d %d %d, full search %d %d %d %d\n", nx, ny, nz, xper, costs.tail, sms,
                                        a.warps, a.th, a.zchunk, a.grid, b.warps, b.th, b.zchunk, b.grid);
         }
     }
