@@ -741,8 +741,8 @@ int launch_normals(tslb_ctx* c) {
 }
 
 // The step kernel on one lattice (shared by the context and the no-alloc
-// paths): the instantiation for the mode, storage, x alignment, tau
-// correction and solid mask of `a`.  launch = false only sets its shared
+// paths): the instantiation for the mode, storage, boundary
+// nodes, tau correction and solid mask of `a`.  launch = false only sets its shared
 // memory attribute.  Returns the error of that attribute; launch errors are
 // left to cudaGetLastError.
 cudaError_t launch_step_kernel(const StepArgs& a, int mode, int prec, cudaStream_t st, bool launch = true,
@@ -1912,7 +1912,7 @@ void ens_plan(tslb_ensemble* e) {
     }
 }
 
-// The ensemble kernel of the ensemble's mode, storage and x alignment:
+// The ensemble kernel of the ensemble's mode, storage and boundary nodes:
 // sets its shared-memory attribute and (launch) launches one step.
 cudaError_t ens_kernel(tslb_ensemble* e, bool launch) {
     const int grid = e->grid > 0 ? std::min(e->grid, e->nwork) : e->nwork;

@@ -35,18 +35,20 @@
 // exist in memory.
 //
 // What bounds it: the latency of the chain through a plane, not HBM.  On the
-// 384 x 192 x 128 colour channel (FP32) a step takes 0.33 ms on a B200, where
-// the kernel that pulled 27 populations took 0.45 ms (1109 thread instructions
-// a node, issue active 62%) and 88 B a node at the measured copy rate take
-// 0.129 ms.  A warp spends 572 instructions on a row and plane (640 a target
-// node with the rims), issue is active 58% of the cycles; the stalls are spread
-// over shared-memory and shuffle latency, fixed instruction latency and the
-// plane barrier.  So registers buy more than instructions: 16 warps of 128
-// registers an SM without a spill (a spilled word comes back from L2, as shared
-// memory leaves little L1: 24 bytes of spills in the plane loop cost 12%); two
-// rows a thread on paired FP32 instructions needs 5/7 of the instructions a row
-// but 255 registers, and 8 warps an SM were slower (0.51 ms), 12 with spills
-// slower still (0.66 ms).
+// 384 x 192 x 128 colour channel (FP32, 8-warp blocks) a step takes 0.326 ms on a
+// B200, where the kernel that pulled 27 populations took 0.45 ms (1109 thread
+// instructions a node, issue active 62%) and 88 B a node at the measured copy rate
+// take 0.129 ms.  It executes 794 thread instructions a node, rims included
+// (30 of 32 lanes and 6 of 8 rows are targets), issue is active 62% of the cycles;
+// the stalls are spread over shared-memory and shuffle latency, fixed instruction
+// latency and the plane barrier.  So registers buy more than instructions: 16
+// warps of 128 registers an SM, without a spill in every kernel of a lattice whose
+// boundary nodes have closed sums (a spilled word comes back from L2, as shared
+// memory leaves little L1: 24 bytes of spills in the plane loop cost 12%; the
+// kernels with the other boundary paths, GEN > 0, have up to 90 bytes in some
+// storage forms); two rows a thread on paired FP32 instructions needs 5/7 of the
+// instructions a row but 255 registers, and 8 warps an SM were slower (0.51 ms),
+// 12 with spills slower still (0.66 ms).
 #pragma once
 
 #include "step_plan.h"

@@ -387,7 +387,9 @@ const char* tslb_ensemble_last_error(tslb_ensemble* e);
  * f at d_x + f * field_stride (floats), x fastest, field 0 = rho - 1, then
  * u, v, w, pxx, pxy, pxz, pyy, pyz, pzz, phi.  Both 16-byte aligned,
  * field_stride >= nx*ny*nz and a multiple of 4; the two ranges of
- * 11 * field_stride floats must not overlap.  Inlet faces are not supported
+ * 11 * field_stride floats must not overlap.  The step may be launched while
+ * the kernel before it on the stream still runs, and waits on the device for
+ * that kernel to complete before it touches the buffers.  Inlet faces are not supported
  * (their planes need storage).  The work is queued on `stream`
  * (cudaStream_t, NULL = default stream) and not waited for.  A step that
  * produces a non-finite moment sets the flag; read it with
