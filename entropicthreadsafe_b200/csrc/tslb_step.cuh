@@ -213,7 +213,8 @@ struct Strided {
 // listed, and the block's warps share them, half a warp a node and a lane a
 // direction (9 at a face, 15 at an edge, 19 at a corner): 160 x 128 x 96
 // colour steps with outlets normal to x / edges of bounce-back and moving walls took
-// 941 / 821 us in turn and take 195 / 179 us.
+// 941 / 821 us in turn and take 191 / 177 us.
+
 // The directions, as bits of a 3 x 3 x 3 index, whose source lies behind one of the
 // faces of mask.
 __device__ __forceinline__ unsigned directions_behind(unsigned mask) {
